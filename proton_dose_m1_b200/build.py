@@ -16,7 +16,7 @@ ROOT = PKG.parent
 LIB = PKG / "libpdm1.so"
 CSRC = PKG / "csrc"
 BUILD = PKG / "_build"
-HEADERS = [CSRC / "pdm1_math.cuh", CSRC / "pdm1_device.cuh", CSRC / "pdm1_stage.cuh",
+HEADERS = [CSRC / "pdm1_math.cuh", CSRC / "pdm1_fp64.cuh", CSRC / "pdm1_device.cuh", CSRC / "pdm1_stage.cuh",
            ROOT / "include" / "pdm1.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off"]

@@ -5,6 +5,7 @@
 
 #include "../../include/pdm1.h"
 #include "pdm1_math.cuh"
+#include "pdm1_fp64.cuh"
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -32,6 +33,9 @@ struct BoxModelDev {
 };
 
 int pack_box_model(const pdm1_box_model *m, BoxModelDev &out);
+
+// Spacings whose quotients pdm1_fp64.cuh may take without the IEEE routine.
+inline bool near_spacing(double h) { return h >= 0x1p-200 && h <= 0x1p200; }
 
 enum { ERR_DEV_RANGE = 1, ERR_DEV_MAXSTEPS = 2, ERR_DEV_NONFINITE = 4, ERR_DEV_CAPACITY = 8, ERR_DEV_TIMEOUT = 16 };
 // ---------------------------------------------------------------------------
@@ -75,6 +79,8 @@ struct MarchSummary {
 struct ConfigDev {
     int nx, ny, nz;
     double dx, dy, dz;
+    double inv_dx, inv_dy, inv_dz;   // their reciprocals, for the divergence
+    int spacing_near;                // the spacings are in the range of quotient()
     int nm;
     int scattering, nuclear, interp, scheme, unit_speeds;
     int cfl_floor;       // moving box: CFL bound at least the phantom's vacuum bound
@@ -371,7 +377,8 @@ __device__ __forceinline__ double cfl_term(const ConfigDev &cf, double rf, const
     } else {
         const T p = T(u[0]), x = T(u[1]), y = T(u[2]), z = T(u[3]);
         T a[3];
-        max_abs_speeds3(p, x, y, z, a);
+        if constexpr (sizeof(T) == sizeof(double)) speeds3_64(u, a);
+        else max_abs_speeds3(p, x, y, z, a);
         a0 = double(a[0]);
         a1 = double(a[1]);
         a2 = double(a[2]);
@@ -385,7 +392,14 @@ __device__ __forceinline__ double cfl_term(const ConfigDev &cf, double rf, const
     if (!use[0]) a0 = 0.0;
     if (!use[1]) a1 = 0.0;
     if (!use[2]) a2 = 0.0;
-    return a0 / (s * cf.dx) + a1 / (s * cf.dy) + a2 / (s * cf.dz);
+    const double b0 = s * cf.dx, b1 = s * cf.dy, b2 = s * cf.dz;
+    if constexpr (sizeof(T) == sizeof(double)) {
+        // speeds are 0 (masked) or above 1e-6, so the quotients are in range when the divisors are
+        auto in = [](double b) { return abs_hi(b) - exp_word(-200) < exp_word(200) - exp_word(-200); };
+        if (in(b0) && in(b1) && in(b2) && a0 <= 2.0 && a1 <= 2.0 && a2 <= 2.0)
+            return quotient(a0, b0, rcp_near(b0)) + quotient(a1, b1, rcp_near(b1)) + quotient(a2, b2, rcp_near(b2));
+    }
+    return a0 / b0 + a1 / b1 + a2 / b2;
 }
 
 template <int THREADS = NT>

@@ -1117,6 +1117,8 @@ int create_plan(const pdm1_problem *problem, const pdm1_beam *beams, int nbeams,
     cf.tile = kTiles[0];
     cf.tile_id = 0;
     cf.dx = p.dx; cf.dy = p.dy; cf.dz = p.dz;
+    cf.inv_dx = 1.0 / p.dx; cf.inv_dy = 1.0 / p.dy; cf.inv_dz = 1.0 / p.dz;
+    cf.spacing_near = near_spacing(p.dx) && near_spacing(p.dy) && near_spacing(p.dz);
     cf.nm = p.n_materials;
     cf.spatial = p.spatial_scheme;
     cf.stencil_radius = ghost_width(p.spatial_scheme);
@@ -1899,6 +1901,8 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
     cf.tile = kTiles[0];
     cf.tile_id = 0;
     cf.dx = p.dx; cf.dy = p.dy; cf.dz = p.dz;
+    cf.inv_dx = 1.0 / p.dx; cf.inv_dy = 1.0 / p.dy; cf.inv_dz = 1.0 / p.dz;
+    cf.spacing_near = near_spacing(p.dx) && near_spacing(p.dy) && near_spacing(p.dz);
     cf.nm = p.n_materials;
     cf.spatial = p.spatial_scheme;
     cf.stencil_radius = ghost_width(p.spatial_scheme);

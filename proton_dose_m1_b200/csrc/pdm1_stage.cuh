@@ -147,6 +147,7 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
     constexpr int NF = Tl::NF, NFX = Tl::NFX, NFY = Tl::NFY;
     constexpr int SX = Tl::SX, SY = Tl::SY, SZ = Tl::SZ;
     constexpr int AX = Tl::AX, AY = Tl::AY, AZ = Tl::AZ;
+    constexpr bool kNear = sizeof(T) == sizeof(double);   // pdm1_fp64.cuh's branch-free face path
     const ConfigDev &cf = *a.cf;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *smem = reinterpret_cast<T *>(smem_raw);
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
         const int i0 = tx * TX, j0 = ty * TY, k0 = tz * TZ;
 
         // ---- 1. stage the stencil source + halo (the core into all three arms) ----
+        int out_of_range = 0;   // a staged value lies outside weno_range
         if constexpr (kF4Source<T, MODE>) {
             // the float4 stage state: bulk copies, or (bulk_stage == 0) one
             // 128-bit load per cell; the arms receive the same values either way
@@ -244,6 +246,7 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const T v = T(u[c]);
+                if constexpr (kNear) out_of_range |= !weno_range(u[c]);
                 arm_at(s.X, AX, c, ex) = v;
                 if (core) {
                     arm_at(s.Y, AY, c, ey) = v;
@@ -258,7 +261,10 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
             double u[4];
             load_cell<MODE>(cf, co, d, src, i0 + i, gj, k0 + k, u);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) arm_at(s.Y, AY, c, (i * (TY + 6) + aj) * TZ + k) = T(u[c]);
+            for (int c = 0; c < 4; ++c) {
+                if constexpr (kNear) out_of_range |= !weno_range(u[c]);
+                arm_at(s.Y, AY, c, (i * (TY + 6) + aj) * TZ + k) = T(u[c]);
+            }
         }
         for (int e = tid; e < SZ; e += NT) {
             int kk = e % 6, j = (e / 6) % TY, i = e / (6 * TY);
@@ -268,10 +274,15 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
             double u[4];
             load_cell<MODE>(cf, co, d, src, i0 + i, j0 + j, gk, u);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) arm_at(s.Z, AZ, c, (i * TY + j) * (TZ + 6) + ak) = T(u[c]);
+            for (int c = 0; c < 4; ++c) {
+                if constexpr (kNear) out_of_range |= !weno_range(u[c]);
+                arm_at(s.Z, AZ, c, (i * TY + j) * (TZ + 6) + ak) = T(u[c]);
+            }
         }
         }   // the double-precision source
-        __syncthreads();
+        bool ieee = false;   // the tile's reconstructions take the IEEE path
+        if constexpr (kNear) ieee = __syncthreads_or(out_of_range) != 0;
+        else __syncthreads();
         // ---- 2. z-min ghost cells: quartic extrapolation through the inflow ----
         if (k0 == 0) {
             for (int e = tid; e < 4 * TX * TY; e += NT) {
@@ -292,8 +303,10 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
                     z(2) = T(3.0) * ui - T(2.5) * u0 + T(0.5) * u1;
                     z(1) = T(9.0) * ui - T(10.5) * u0 + T(2.5) * u1;
                 }
+                if constexpr (kNear) out_of_range |= !(weno_range(z(0)) && weno_range(z(1)) && weno_range(z(2)));
             }
-            __syncthreads();
+            if constexpr (kNear) ieee = __syncthreads_or(out_of_range) != 0;
+            else __syncthreads();
         }
         // ---- 3. every face of the tile: WENO-Z, projection, HLL ----
         for (int f = tid; f < NF; f += NT) {
@@ -344,8 +357,12 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
                         T w[6];
 #pragma unroll
                         for (int q = 0; q < 6; ++q) w[q] = base[c * cs + q * stride];
-                        L[c] = weno_left(w[0], w[1], w[2], w[3], w[4]);
-                        R[c] = weno_left(w[5], w[4], w[3], w[2], w[1]);
+                        if (ieee) {
+                            L[c] = weno_left_ieee(w[0], w[1], w[2], w[3], w[4]);
+                            R[c] = weno_left_ieee(w[5], w[4], w[3], w[2], w[1]);
+                        } else {
+                            weno_pair(w, L[c], R[c]);
+                        }
                     }
                 }
             } else {
@@ -362,22 +379,23 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
                         L[c] = hi;
                         muscl_faces(w0, w1, wp, lo, hi);
                         R[c] = lo;
-                    } else {   // WENO3, weno3.py:108-171
+                    } else if constexpr (kNear) {   // WENO3, weno3.py:108-171
+                        L[c] = ieee ? weno3_left_ieee(wm, w0, w1) : weno3_near(wm, w0, w1);
+                        R[c] = ieee ? weno3_left_ieee(wp, w1, w0) : weno3_near(wp, w1, w0);
+                    } else {
                         L[c] = weno3_left(wm, w0, w1);
                         R[c] = weno3_left(wp, w1, w0);
                     }
                 }
             }
-            T F[4];
-            if constexpr (sizeof(T) == sizeof(float)) {
-                face_flux_f32x2(L, R, axis, unit, F);
+            if constexpr (kNear) {
+                face_flux64(L, R, axis, unit, s.F + f, NF);
             } else {
-                project(L[0], L[1], L[2], L[3]);
-                project(R[0], R[1], R[2], R[3]);
-                hll_flux(L, R, axis, unit, F);
-            }
+                T F[4];
+                face_flux_f32x2(L, R, axis, unit, F);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) s.F[c * NF + f] = F[c];
+                for (int c = 0; c < 4; ++c) s.F[c * NF + f] = F[c];
+            }
         }
         __syncthreads();
         // ---- 4. divergence and the stage update, one cell per thread ----
@@ -394,10 +412,20 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
                 const T *F = s.F + c * NF;
-                T gx = (F[fx1] - F[fx0]) / T(cf.dx);
-                T gy = (F[fy1] - F[fy0]) / T(cf.dy);
-                T gz = (F[fz1] - F[fz0]) / T(cf.dz);
-                L[c] = double(-(gx + gy + gz));
+                const T ex = F[fx1] - F[fx0], ey = F[fy1] - F[fy0], ez = F[fz1] - F[fz0];
+                if constexpr (kNear) {
+                    // spacings are in range (checked with the plan); a difference that is not: IEEE
+                    double gx = quotient(ex, cf.dx, cf.inv_dx), gy = quotient(ey, cf.dy, cf.inv_dy);
+                    double gz = quotient(ez, cf.dz, cf.inv_dz);
+                    if (!(cf.spacing_near && zero_or_within<-900, 700>(ex) && zero_or_within<-900, 700>(ey) &&
+                          zero_or_within<-900, 700>(ez))) {
+                        gx = div_ieee(ex, cf.dx); gy = div_ieee(ey, cf.dy); gz = div_ieee(ez, cf.dz);
+                    }
+                    L[c] = -(gx + gy + gz);
+                } else {
+                    const T gx = ex / T(cf.dx), gy = ey / T(cf.dy), gz = ez / T(cf.dz);
+                    L[c] = double(-(gx + gy + gz));
+                }
             }
             const size_t o = ((size_t)li * ny + lj) * nz + lk;
             if (MODE == MODE_RHS) {
@@ -425,10 +453,10 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
                         double v0 = s0 * un[c];
                         double v = L[c] * dE + v0;
                         v1[c] = v;
-                        double w = v * (c == 0 ? co.c1p[m] : co.c1c[m]);
-                        u1[c] = w / co.S1[m];
+                        u1[c] = v * (c == 0 ? co.c1p[m] : co.c1c[m]);
                     }
-                    project(u1[0], u1[1], u1[2], u1[3]);
+                    div4(u1, co.S1[m]);
+                    project64(u1);
                     if constexpr (kF4Dest<T, MODE>)
                         reinterpret_cast<float4 *>(U1)[o] = make_float4(float(u1[0]), float(u1[1]), float(u1[2]),
                                                                         float(u1[3]));
@@ -447,10 +475,10 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
                         r = (r * dE + Vb[c * N + o]) * 0.25;
                         double v = 0.75 * (s0 * un[c]) + r;
                         Vb[c * N + o] = v;
-                        double w = v * (c == 0 ? co.c2p[m] : co.c2c[m]);
-                        u2[c] = w / co.S2[m];
+                        u2[c] = v * (c == 0 ? co.c2p[m] : co.c2c[m]);
                     }
-                    project(u2[0], u2[1], u2[2], u2[3]);
+                    div4(u2, co.S2[m]);
+                    project64(u2);
                     if constexpr (kF4Dest<T, MODE>) {
                         reinterpret_cast<float4 *>(U2)[o] = make_float4(float(u2[0]), float(u2[1]), float(u2[2]),
                                                                         float(u2[3]));
@@ -471,10 +499,10 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
                             double r = L[c] * (c == 0 ? co.c2ip[m] : co.c2ic[m]);
                             r = (r * dE + Vb[c * N + o]) * (2.0 / 3.0);
                             double v = 1.0 / 3.0 * (s0 * un[c]) + r;
-                            double w = v * (c == 0 ? co.c1p[m] : co.c1c[m]);
-                            unew[c] = w / co.S1[m];
+                            unew[c] = v * (c == 0 ? co.c1p[m] : co.c1c[m]);
                         }
-                        project(unew[0], unew[1], unew[2], unew[3]);
+                        div4(unew, co.S1[m]);
+                        project64(unew);
                         if constexpr (sizeof(T) == sizeof(double)) {
                             double u2c = double(s.X[((0 * (TX + 6) + (i + 3)) * TY + j) * TZ + k]);
                             double q2 = u2c * co.S2[m];
@@ -485,10 +513,10 @@ __global__ void __launch_bounds__(Tl::NT, (sizeof(T) == sizeof(double) ? 2 : 4) 
                     } else {   // forward Euler, numerics/energy.py:663-722
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
-                            double w = L[c] * dE + s0 * un[c];
-                            unew[c] = w / co.S1[m];
+                            unew[c] = L[c] * dE + s0 * un[c];
                         }
-                        project(unew[0], unew[1], unew[2], unew[3]);
+                        div4(unew, co.S1[m]);
+                        project64(unew);
                         ed = dE * un[0] * s0;
                     }
                     if (cf.strang) {
