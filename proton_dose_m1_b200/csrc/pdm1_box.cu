@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(NT) box_moments_kernel(const ConfigDev *cfp, c
         const int i0 = tx * TX, j0 = ty * TY, k0 = tz * TZ;
         const int ii = tid / (TY * TZ), jj = (tid / TZ) % TY, kk = tid % TZ;
         const int li = i0 + ii, lj = j0 + jj, lk = k0 + kk;
-        const bool valid = li < d.nx && lj < d.ny && lk < d.nz;
+        const bool valid = tid < TX * TY * TZ && li < d.nx && lj < d.ny && lk < d.nz;
         double u[4] = {0.0, 0.0, 0.0, 0.0};
         if (valid) {
             const size_t N = (size_t)d.nx * d.ny * d.nz, o = ((size_t)li * d.ny + lj) * d.nz + lk;

@@ -54,12 +54,14 @@ struct DomainDev {
     int tx, ty, tz;          // tile shape of the stage kernels
     int tiles_y, tiles_z, ntiles;
     int inflow;              // the domain's z-min face is the beam entrance (k0 == 0)
+    int small;               // the tiles are SmallTile's
 };
 
-// Tile shape (cells) of the stage kernels; every shape holds one cell per
-// thread of a 256-thread CTA.
+// Tile shape (cells) of the stage kernels, one cell per thread of a 256-thread
+// CTA; a domain of at most `small` tiles of 4x4x4 cells takes those instead.
 struct TileDims {
     int x, y, z;
+    int small;
 };
 
 // One pencil beam of a march (numerics/boundary.py:63-114): spectrum, angular
@@ -225,7 +227,7 @@ __device__ __forceinline__ void source_factor(double ts, double tn, bool inverse
 // ---------------------------------------------------------------------------
 // The fused stage kernel
 // ---------------------------------------------------------------------------
-constexpr int NT = 256;   // threads of a stage CTA = cells of a tile
+constexpr int NT = 256;   // threads of a stage CTA
 
 // A tile shape: the tile's cells, its cross-shaped 3-cell WENO halo (no
 // corners: WENO reads along one axis at a time) and its faces.  Shared memory
@@ -234,8 +236,8 @@ constexpr int NT = 256;   // threads of a stage CTA = cells of a tile
 // one arm.
 template <int X, int Y, int Z>
 struct Tile {
-    static constexpr int NT = X * Y * Z;   // threads of the CTA: one cell each
-    static_assert(NT == 256 || NT == 512, "256- or 512-cell tiles");
+    static constexpr int CELLS = X * Y * Z;
+    static_assert(CELLS <= NT, "at most one cell per thread");
     static constexpr int TX = X, TY = Y, TZ = Z;
     static constexpr int NFX = (X + 1) * Y * Z, NFY = X * (Y + 1) * Z, NFZ = X * Y * (Z + 1);
     static constexpr int NF = NFX + NFY + NFZ;
@@ -246,7 +248,7 @@ struct Tile {
     static constexpr int AY = X * (Y + 6) * Z;
     static constexpr int AZ = X * Y * (Z + 6);
     template <typename T>
-    static constexpr size_t smem_bytes() { return sizeof(T) * 4 * (AX + AY + AZ + NF); }
+    static constexpr size_t arm_bytes() { return sizeof(T) * 4 * (AX + AY + AZ + NF); }
 };
 
 // The tile shapes the stage kernels are built for, the autotuner's candidates.
@@ -257,14 +259,29 @@ constexpr int kNumTiles = 3;
 using Tile0 = Tile<4, 8, 8>;
 using Tile1 = Tile<8, 8, 4>;
 using Tile2 = Tile<2, 8, 16>;
-constexpr TileDims kTiles[kNumTiles] = {{4, 8, 8}, {8, 8, 4}, {2, 8, 16}};
+constexpr TileDims kTiles[kNumTiles] = {{4, 8, 8, 0}, {8, 8, 4, 0}, {2, 8, 16, 0}};
 constexpr int kMaxTileZ = 16;
+// A domain whose 4x4x4 tiles all fit one wave of the resident CTAs takes them:
+// 240 faces for 256 threads, one round instead of the 4x8x8 tile's three and a
+// half, and four times the CTAs.  Measured, one FP64 energy step: 225 small tiles
+// (12x12x100) 175 -> 118 us; 480 (16x16x120, two waves) 143 -> 153 us, so the line
+// lies at one wave.  FP32 form, four CTAs per SM: 480 small tiles 132 -> 101 us; 875
+// (1.5 waves) 116 -> 126 us.
+using SmallTile = Tile<4, 4, 4>;
+inline TileDims with_small(TileDims t, int slots, int nbeams) {
+    t.small = slots / nbeams;
+    return t;
+}
 
 __host__ __device__ inline DomainDev make_domain(int i0, int j0, int k0, int nx, int ny, int nz, int inflow,
                                                  TileDims t) {
     DomainDev d;
     d.i0 = i0; d.j0 = j0; d.k0 = k0;
     d.nx = nx; d.ny = ny; d.nz = nz;
+    using S = SmallTile;
+    const long long n_small = (long long)((nx + S::TX - 1) / S::TX) * ((ny + S::TY - 1) / S::TY) * ((nz + S::TZ - 1) / S::TZ);
+    d.small = n_small <= t.small;
+    if (d.small) t = TileDims{S::TX, S::TY, S::TZ, t.small};
     d.tx = t.x; d.ty = t.y; d.tz = t.z;
     d.tiles_y = (ny + t.y - 1) / t.y;
     d.tiles_z = (nz + t.z - 1) / t.z;

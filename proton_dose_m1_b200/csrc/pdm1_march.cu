@@ -904,8 +904,8 @@ int cell_blocks(const pdm1_plan *pl) {
 
 template <class Tl>
 void launch_stage64(int mode, int grid, const StageArgs &a, cudaStream_t stream) {
-    const size_t bytes = Tl::template smem_bytes<double>();
-    constexpr int nt = Tl::NT;
+    const size_t bytes = stage_smem_bytes<double, Tl>();
+    constexpr int nt = NT;
     switch (mode) {
     case MODE_A: stage_kernel<double, MODE_A, Tl><<<grid, nt, bytes, stream>>>(a); break;
     case MODE_B: stage_kernel<double, MODE_B, Tl><<<grid, nt, bytes, stream>>>(a); break;
@@ -995,7 +995,7 @@ int launch_step(pdm1_plan *pl, const StageArgs &a, double *energies, cudaStream_
 
 template <class Tl>
 cudaError_t set_attributes64() {
-    const int bytes = (int)Tl::template smem_bytes<double>();
+    const int bytes = (int)stage_smem_bytes<double, Tl>();
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(stage_kernel<double, MODE_A, Tl>, attr, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(stage_kernel<double, MODE_B, Tl>, attr, bytes);
@@ -1085,14 +1085,16 @@ void destroy_plan(pdm1_plan *pl) {
 }
 
 // Persistent grid of the stage kernels: resident CTAs per SM x SMs, capped by
-// the tiles of the full grid.  256-cell tiles: 2 CTAs per SM in double, 4 in
-// float (64 registers; 4 x 256 threads hide more of the MUFU and shared-memory
-// latency than 3 x 256 at 80 registers: -4 % stage time on field256); a
-// 512-cell tile holds half as many CTAs.
+// the tiles of the full grid.  2 CTAs per SM in double, 4 in float (64 registers;
+// 4 x 256 threads hide more of the MUFU and shared-memory latency than 3 x 256 at
+// 80 registers: -4 % stage time on field256).
+int stage_slots(const pdm1_problem &p, int sms) { return (p.precision == PDM1_FP32_FP64 ? 4 : 2) * sms; }
+
 int stage_grid(const pdm1_problem &p, TileDims t, int nbeams, int sms) {
-    const int per_sm = (p.precision == PDM1_FP32_FP64 ? 4 : 2) * 256 / (t.x * t.y * t.z);
-    size_t tiles = (size_t)make_domain(0, 0, 0, p.nx, p.ny, p.nz, 1, t).ntiles * nbeams;
-    return (int)std::max<size_t>(1, std::min<size_t>(tiles, (size_t)std::max(1, per_sm) * sms));
+    // a moving box may take small tiles where the full grid does not
+    const size_t tiles = std::max<size_t>(make_domain(0, 0, 0, p.nx, p.ny, p.nz, 1, t).ntiles,
+                                          p.moving_active_domain ? t.small : 0) * nbeams;
+    return (int)std::max<size_t>(1, std::min<size_t>(tiles, stage_slots(p, sms)));
 }
 
 // A plan for `nbeams` beams on one phantom; every beam's buffers hold `cap` cells.
@@ -1114,7 +1116,12 @@ int create_plan(const pdm1_problem *problem, const pdm1_beam *beams, int nbeams,
     std::vector<std::pair<size_t, int>> fix;
     ConfigDev &cf = pl->cf;
     cf.nx = p.nx; cf.ny = p.ny; cf.nz = p.nz;
-    cf.tile = kTiles[0];
+    {
+        int dev = 0, sms = 148;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        pl->sms = sms;
+    }
+    cf.tile = with_small(kTiles[0], stage_slots(p, pl->sms), nbeams);
     cf.tile_id = 0;
     cf.dx = p.dx; cf.dy = p.dy; cf.dz = p.dz;
     cf.inv_dx = 1.0 / p.dx; cf.inv_dy = 1.0 / p.dy; cf.inv_dz = 1.0 / p.dz;
@@ -1238,15 +1245,7 @@ int create_plan(const pdm1_problem *problem, const pdm1_beam *beams, int nbeams,
     cf.plane = pl->d_plane;
     cf.rec = nullptr;
     cf.rec_max = 0;
-    {
-        int dev = 0, sms = 148;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        // resident CTAs per SM of the stage kernel: 2 in double, 4 in float
-        // (64 registers; 4 x 256 threads hide more of the MUFU and shared-memory
-        // latency than 3 x 256 at 80 registers: -4 % stage time on field256)
-        pl->sms = sms;
-        cf.grid_ctas = stage_grid(p, cf.tile, B, sms);
-    }
+    cf.grid_ctas = stage_grid(p, cf.tile, B, pl->sms);
     bool ok = cudaMemcpy(pl->d_tables, blob.data(), blob.size() * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(pl->d_ids, problem->ids, N * sizeof(int32_t), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(pl->d_beams, pl->h_beams.data(), B * sizeof(BeamDev), cudaMemcpyHostToDevice) == cudaSuccess &&
@@ -1468,7 +1467,7 @@ int pdm1_tile_shape(int tile_id, int *tx, int *ty, int *tz) {
 int pdm1_plan_set_tile(pdm1_plan *pl, int tile_id) {
     if (!pl) return set_error(PDM1_ERR_ARGUMENT, "plan is NULL");
     if (tile_id < 0 || tile_id >= kNumTiles) return set_error(PDM1_ERR_ARGUMENT, "unknown tile shape");
-    const TileDims t = kTiles[tile_id];
+    const TileDims t = with_small(kTiles[tile_id], stage_slots(pl->p, pl->sms), pl->nbeams);
     pl->cf.tile = t;
     pl->cf.tile_id = tile_id;
     pl->cf.grid_ctas = stage_grid(pl->p, t, pl->nbeams, pl->sms);
@@ -1798,14 +1797,14 @@ void launch_step_plain(const pdm1_problem &p, ConfigDev *d_cf, Coeffs *d_co, Mar
                        const StageArgs &a, double *energies, int tiles, cudaStream_t stream) {
     prologue_kernel<<<1, 256, 0, stream>>>(d_cf, d_co, d_st, energies);
     if (p.energy_scheme == PDM1_SCHEME_FORWARD_EULER) {
-        stage_kernel<double, MODE_EULER, Tile0><<<tiles, NT, Tile0::smem_bytes<double>(), stream>>>(a);
+        stage_kernel<double, MODE_EULER, Tile0><<<tiles, NT, stage_smem_bytes<double, Tile0>(), stream>>>(a);
         const size_t N = (size_t)p.nx * p.ny * p.nz;
         euler_finish_kernel<<<(int)std::max<size_t>(1, std::min<size_t>((N + NT - 1) / NT, 148 * 8)), NT, 0, stream>>>(a);
         return;
     }
-    stage_kernel<double, MODE_A, Tile0><<<tiles, NT, Tile0::smem_bytes<double>(), stream>>>(a);
-    stage_kernel<double, MODE_B, Tile0><<<tiles, NT, Tile0::smem_bytes<double>(), stream>>>(a);
-    stage_kernel<double, MODE_C, Tile0><<<tiles, NT, Tile0::smem_bytes<double>(), stream>>>(a);
+    stage_kernel<double, MODE_A, Tile0><<<tiles, NT, stage_smem_bytes<double, Tile0>(), stream>>>(a);
+    stage_kernel<double, MODE_B, Tile0><<<tiles, NT, stage_smem_bytes<double, Tile0>(), stream>>>(a);
+    stage_kernel<double, MODE_C, Tile0><<<tiles, NT, stage_smem_bytes<double, Tile0>(), stream>>>(a);
 }
 
 }  // namespace
@@ -1882,10 +1881,10 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
     if (!g_noalloc_base[dev]) {
         void *ptr = nullptr;
         CUDA_TRY(cudaGetSymbolAddress(&ptr, g_noalloc_scratch));
-        CUDA_TRY(cudaFuncSetAttribute(stage_kernel<double, MODE_A, Tile0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile0::smem_bytes<double>()));
-        CUDA_TRY(cudaFuncSetAttribute(stage_kernel<double, MODE_B, Tile0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile0::smem_bytes<double>()));
-        CUDA_TRY(cudaFuncSetAttribute(stage_kernel<double, MODE_C, Tile0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile0::smem_bytes<double>()));
-        CUDA_TRY(cudaFuncSetAttribute(stage_kernel<double, MODE_EULER, Tile0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Tile0::smem_bytes<double>()));
+        CUDA_TRY(cudaFuncSetAttribute(stage_kernel<double, MODE_A, Tile0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem_bytes<double, Tile0>()));
+        CUDA_TRY(cudaFuncSetAttribute(stage_kernel<double, MODE_B, Tile0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem_bytes<double, Tile0>()));
+        CUDA_TRY(cudaFuncSetAttribute(stage_kernel<double, MODE_C, Tile0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem_bytes<double, Tile0>()));
+        CUDA_TRY(cudaFuncSetAttribute(stage_kernel<double, MODE_EULER, Tile0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)stage_smem_bytes<double, Tile0>()));
         g_noalloc_base[dev] = ptr;
     }
     unsigned char *base = static_cast<unsigned char *>(g_noalloc_base[dev]);
@@ -1898,7 +1897,9 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
     // the configuration, tables, ids and inflow profile go into the scratch array
     ConfigDev cf{};
     cf.nx = p.nx; cf.ny = p.ny; cf.nz = p.nz;
-    cf.tile = kTiles[0];
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cf.tile = with_small(kTiles[0], stage_slots(p, sms), 1);
     cf.tile_id = 0;
     cf.dx = p.dx; cf.dy = p.dy; cf.dz = p.dz;
     cf.inv_dx = 1.0 / p.dx; cf.inv_dy = 1.0 / p.dy; cf.inv_dz = 1.0 / p.dz;
@@ -1923,11 +1924,7 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
     cf.step_limit = -1;
     cf.n_targets = 0;
     cf.targets = nullptr;
-    {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cf.grid_ctas = std::max(1, std::min(make_domain(0, 0, 0, p.nx, p.ny, p.nz, 1, kTiles[0]).ntiles, 2 * sms));
-    }
+    cf.grid_ctas = stage_grid(p, cf.tile, 1, sms);
     cf.ids = reinterpret_cast<const int32_t *>(base + o_ids);
     cf.nbeams = 1;
     cf.cap = N;
@@ -1939,7 +1936,7 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
     bm.sigma_E = p.energy_spread;
     bm.rf = dd_exp(-(p.angular_spread * p.angular_spread));
     bm.spatial = reinterpret_cast<const double *>(base + o_sp);
-    bm.init_box = make_domain(0, 0, 0, p.nx, p.ny, p.nz, 1, kTiles[0]);
+    bm.init_box = make_domain(0, 0, 0, p.nx, p.ny, p.nz, 1, cf.tile);
     for (int m = 0; m < p.n_materials; ++m) {
         const pdm1_material &mt = p.materials[m];
         const pdm1_table *tabs[3] = {&mt.stopping_power, &mt.transport, &mt.nuclear};

@@ -14,7 +14,7 @@ namespace {
 
 template <class Tl>
 cudaError_t set_attributes() {
-    const int bytes = (int)Tl::template smem_bytes<float>();
+    const int bytes = (int)stage_smem_bytes<float, Tl>();
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     cudaError_t e = cudaFuncSetAttribute(stage_kernel<float, MODE_A, Tl>, attr, bytes);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(stage_kernel<float, MODE_B, Tl>, attr, bytes);
@@ -27,8 +27,8 @@ cudaError_t set_attributes() {
 
 template <class Tl>
 void launch(int mode, int grid, const StageArgs &a, cudaStream_t stream) {
-    const size_t bytes = Tl::template smem_bytes<float>();
-    constexpr int nt = Tl::NT;
+    const size_t bytes = stage_smem_bytes<float, Tl>();
+    constexpr int nt = NT;
     switch (mode) {
     case MODE_A: stage_kernel<float, MODE_A, Tl><<<grid, nt, bytes, stream>>>(a); break;
     case MODE_B: stage_kernel<float, MODE_B, Tl><<<grid, nt, bytes, stream>>>(a); break;
