@@ -54,14 +54,11 @@ struct DomainDev {
     int tx, ty, tz;          // tile shape of the stage kernels
     int tiles_y, tiles_z, ntiles;
     int inflow;              // the domain's z-min face is the beam entrance (k0 == 0)
-    int small;               // the tiles are SmallTile's
 };
 
-// Tile shape (cells) of the stage kernels, one cell per thread of a 256-thread
-// CTA; a domain of at most `small` tiles of 4x4x4 cells takes those instead.
+// Tile shape (cells) of the stage kernels.
 struct TileDims {
     int x, y, z;
-    int small;
 };
 
 // One pencil beam of a march (numerics/boundary.py:63-114): spectrum, angular
@@ -124,6 +121,7 @@ struct ConfigDev {
     float *rec;                 // recorder rows (one-beam full-domain plans), or NULL
     int rec_max;
     double rec_tail_tol[2];     // recorder: the two fluence-tail thresholds
+    double density[kMaxMat];
     MatDev mats[kMaxMat];
 };
 
@@ -180,11 +178,26 @@ __host__ __device__ inline DomainDev make_domain(int i0, int j0, int k0, int nx,
 // ---------------------------------------------------------------------------
 // Material coefficients (device), mirroring physics/*.py
 // ---------------------------------------------------------------------------
-__device__ inline bool stopping_power_dev(const MatDev &m, double E, double &out) {
-    if (!clip_energy(m.sp, E)) return false;
-    if (E == m.sp.E[m.sp.n - 1]) { out = m.sp.v[m.sp.n - 1]; return true; }
-    out = pchip_eval(m.sp, E);
+// A table at E, clipped to it (false: outside): PCHIP or numpy.interp.  The loads of
+// the guessed interval go out together with those of the table's ends; a guess
+// that misses (rounding of the logarithm) takes the general evaluation.
+__device__ inline bool table_dev(const TableView &view, bool pchip, double E, double &out) {
+    const TableView t = view;
+    const int last = t.n - 1;
+    int i = t.inv_log_step > 0.0 && E > 0.0 ? interval_guess(t, E) : search_right(t, E);
+    i = i < 0 ? 0 : (i > last - 1 ? last - 1 : i);
+    const double lo = t.E[0], hi = t.E[last], v_last = t.v[last];
+    const double e0 = t.E[i], e1 = t.E[i + 1], v0 = t.v[i], v1 = t.v[i + 1];
+    const double s0 = t.slope[i], s1 = t.slope[i + 1];
+    if (!clip_energy(lo, hi, E)) return false;
+    if (E >= hi) out = v_last;
+    else if (!(e0 <= E && E < e1)) out = pchip ? pchip_eval(t, E) : linear_eval(t, E);
+    else out = pchip ? pchip_interval(e0, e1, v0, v1, s0, s1, E) : linear_interval(e0, e1, v0, v1, E);
     return true;
+}
+
+__device__ inline bool stopping_power_dev(const MatDev &m, double E, double &out) {
+    return table_dev(m.sp, true, E, out);
 }
 
 __device__ inline bool transport_dev(const ConfigDev &cf, const MatDev &m, double E, double &out) {
@@ -197,15 +210,11 @@ __device__ inline bool transport_dev(const ConfigDev &cf, const MatDev &m, doubl
         out = r * r / m.X0;
         return true;
     }
-    if (!clip_energy(m.tr, E)) return false;
-    out = cf.interp == PDM1_INTERP_LINEAR ? linear_eval(m.tr, E) : pchip_eval(m.tr, E);
-    return true;
+    return table_dev(m.tr, cf.interp != PDM1_INTERP_LINEAR, E, out);
 }
 
 __device__ inline bool nuclear_dev(const ConfigDev &cf, const MatDev &m, double E, double &out) {
-    if (!clip_energy(m.nuc, E)) return false;
-    out = cf.interp == PDM1_INTERP_LINEAR ? linear_eval(m.nuc, E) : pchip_eval(m.nuc, E);
-    return true;
+    return table_dev(m.nuc, cf.interp != PDM1_INTERP_LINEAR, E, out);
 }
 
 // numerics/boundary.py:82-114 spectrum factor
@@ -259,29 +268,24 @@ constexpr int kNumTiles = 3;
 using Tile0 = Tile<4, 8, 8>;
 using Tile1 = Tile<8, 8, 4>;
 using Tile2 = Tile<2, 8, 16>;
-constexpr TileDims kTiles[kNumTiles] = {{4, 8, 8, 0}, {8, 8, 4, 0}, {2, 8, 16, 0}};
+constexpr TileDims kTiles[kNumTiles] = {{4, 8, 8}, {8, 8, 4}, {2, 8, 16}};
 constexpr int kMaxTileZ = 16;
-// A domain whose 4x4x4 tiles all fit one wave of the resident CTAs takes them:
-// 240 faces for 256 threads, one round instead of the 4x8x8 tile's three and a
-// half, and four times the CTAs.  Measured, one FP64 energy step: 225 small tiles
+
+// Plans whose grids all fit one wave of the resident CTAs in 4x4x4 tiles take
+// those: 240 faces for 256 threads, one round instead of the 4x8x8 tile's three and
+// a half, and four times the CTAs.  Measured, one FP64 energy step: 225 small tiles
 // (12x12x100) 175 -> 118 us; 480 (16x16x120, two waves) 143 -> 153 us, so the line
 // lies at one wave.  FP32 form, four CTAs per SM: 480 small tiles 132 -> 101 us; 875
 // (1.5 waves) 116 -> 126 us.
 using SmallTile = Tile<4, 4, 4>;
-inline TileDims with_small(TileDims t, int slots, int nbeams) {
-    t.small = slots / nbeams;
-    return t;
-}
+constexpr int kSmallTileId = kNumTiles;
+constexpr TileDims kSmallTile = {4, 4, 4};
 
 __host__ __device__ inline DomainDev make_domain(int i0, int j0, int k0, int nx, int ny, int nz, int inflow,
                                                  TileDims t) {
     DomainDev d;
     d.i0 = i0; d.j0 = j0; d.k0 = k0;
     d.nx = nx; d.ny = ny; d.nz = nz;
-    using S = SmallTile;
-    const long long n_small = (long long)((nx + S::TX - 1) / S::TX) * ((ny + S::TY - 1) / S::TY) * ((nz + S::TZ - 1) / S::TZ);
-    d.small = n_small <= t.small;
-    if (d.small) t = TileDims{S::TX, S::TY, S::TZ, t.small};
     d.tx = t.x; d.ty = t.y; d.tz = t.z;
     d.tiles_y = (ny + t.y - 1) / t.y;
     d.tiles_z = (nz + t.z - 1) / t.z;
@@ -542,7 +546,7 @@ __device__ __forceinline__ void tile_moments_cta(const ConfigDev &cf, int b, con
 // z = 0), then the first and last x / y / z slab of `d` whose max phi exceeds
 // tol * scale (the plan's tolerance for the moving box), an inflow cell above
 // it joining the k = 0 layer.  Called by all threads of a CTA of 256 (8
-// warps) with `red` = 512 doubles of shared memory; results (local indices,
+// warps) with `red` = 16 doubles of shared memory; results (local indices,
 // hi < 0 when none) in the caller's shared memory.
 __device__ inline void significant_box_cta(const ConfigDev &cf, const BeamDev &bm, const DomainDev &d,
                                            const unsigned long long *slab, double ed, double *red, int *s_lo,
@@ -555,50 +559,51 @@ __device__ inline void significant_box_cta(const ConfigDev &cf, const BeamDev &b
     double m = 0.0, mi = 0.0;
     for (int i = t; i < d.nx; i += 256) m = fmax(m, as_d(sx[i]));
     if (d.inflow)
-        for (int e = t; e < d.nx * d.ny; e += 256) mi = fmax(mi, inflow(e / d.ny, e % d.ny));
-    red[t] = m;
-    red[256 + t] = mi;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-        if (t < w) {
-            red[t] = fmax(red[t], red[t + w]);
-            red[256 + t] = fmax(red[256 + t], red[256 + t + w]);
-        }
-        __syncthreads();
+        for (int i = warp; i < d.nx; i += 8)
+            for (int j = lane; j < d.ny; j += 32) mi = fmax(mi, inflow(i, j));
+    for (int w = 16; w > 0; w >>= 1) {
+        m = fmax(m, __shfl_xor_sync(0xffffffffu, m, w));
+        mi = fmax(mi, __shfl_xor_sync(0xffffffffu, mi, w));
     }
-    if (t == 0) {
-        *s_scale = fmax(red[0], red[256]);
-        for (int q = 0; q < 3; ++q) { s_lo[q] = 0x7fffffff; s_hi[q] = -1; }
-    }
+    if (lane == 0) { red[warp] = m; red[8 + warp] = mi; }
+    if (t < 3) { s_lo[t] = 0x7fffffff; s_hi[t] = -1; }
     __syncthreads();
-    const double scale = *s_scale;
+    m = mi = 0.0;
+    for (int w = 0; w < 8; ++w) { m = fmax(m, red[w]); mi = fmax(mi, red[8 + w]); }
+    const double scale = fmax(m, mi);
+    if (t == 0) *s_scale = scale;
     const double thr = tol * scale;
     // an inflow cell above the threshold exists iff the inflow's maximum is above it
-    const bool inflow_on = d.inflow && red[256] > thr;
+    const bool inflow_on = d.inflow && mi > thr;
     if (scale != 0.0) {
-        // one warp per x slab (y slab): the slab maximum, or any inflow cell of
-        // the slab's entrance row above the threshold
-        for (int i = warp; i < d.nx; i += 8) {
-            bool act = as_d(sx[i]) > thr;
-            if (!act && inflow_on) {
+        // one thread per slab: its maximum above the threshold, or the k = 0 layer under
+        // an inflow above it
+        auto scan = [&](const unsigned long long *sl, int n, int ax, bool first) {
+            for (int base = 32 * warp; base < n; base += 256) {
+                const int i = base + lane;
+                const bool act = i < n && (as_d(sl[i]) > thr || (first && i == 0));
+                const unsigned mask = __ballot_sync(0xffffffffu, act);
+                if (lane == 0 && mask) {
+                    atomicMin(&s_lo[ax], base + __ffs(mask) - 1);
+                    atomicMax(&s_hi[ax], base + 31 - __clz(mask));
+                }
+            }
+        };
+        scan(sx, d.nx, 0, false);
+        scan(sy, d.ny, 1, false);
+        scan(sz, d.nz, 2, inflow_on);
+        if (inflow_on) {
+            // one warp per x slab (y slab): any inflow cell of its entrance row above the threshold
+            for (int i = warp; i < d.nx; i += 8) {
                 bool any = false;
                 for (int j = lane; j < d.ny; j += 32) any = any || inflow(i, j) > thr;
-                act = __any_sync(0xffffffffu, any);
+                if (__any_sync(0xffffffffu, any) && lane == 0) { atomicMin(&s_lo[0], i); atomicMax(&s_hi[0], i); }
             }
-            if (act && lane == 0) { atomicMin(&s_lo[0], i); atomicMax(&s_hi[0], i); }
-        }
-        for (int j = warp; j < d.ny; j += 8) {
-            bool act = as_d(sy[j]) > thr;
-            if (!act && inflow_on) {
+            for (int j = warp; j < d.ny; j += 8) {
                 bool any = false;
                 for (int i = lane; i < d.nx; i += 32) any = any || inflow(i, j) > thr;
-                act = __any_sync(0xffffffffu, any);
+                if (__any_sync(0xffffffffu, any) && lane == 0) { atomicMin(&s_lo[1], j); atomicMax(&s_hi[1], j); }
             }
-            if (act && lane == 0) { atomicMin(&s_lo[1], j); atomicMax(&s_hi[1], j); }
-        }
-        for (int k = t; k < d.nz; k += 256) {
-            const bool act = as_d(sz[k]) > thr || (k == 0 && inflow_on);
-            if (act) { atomicMin(&s_lo[2], k); atomicMax(&s_hi[2], k); }
         }
     }
     __syncthreads();
@@ -606,9 +611,10 @@ __device__ inline void significant_box_cta(const ConfigDev &cf, const BeamDev &b
 
 // Switch a beam to the box `nb` (one thread): the capacity check, the
 // compact-state ping-pong, the spectrum for the CFL bound and, for the
-// vacuum-aware CFL (energy.py:496-537), the max inflow over the new box.
+// vacuum-aware CFL (energy.py:496-537), the max inflow over the new box
+// (`with_pin`; box_kernel takes that with its whole CTA).
 __device__ inline void switch_box(const ConfigDev &cf, const BeamDev &bm, Coeffs *co, MarchState *st, int b,
-                                  DomainDev nb, double ed) {
+                                  DomainDev nb, double ed, bool with_pin = true) {
     const DomainDev d = st->dom;
     bool same = nb.i0 == d.i0 && nb.j0 == d.j0 && nb.k0 == d.k0 && nb.nx == d.nx && nb.ny == d.ny && nb.nz == d.nz;
     if (!same && (size_t)nb.nx * nb.ny * nb.nz > cf.cap) {
@@ -627,7 +633,7 @@ __device__ inline void switch_box(const ConfigDev &cf, const BeamDev &bm, Coeffs
     co->ed_cfl = ed;
     st->newmax_bits = 0ull;
     double pin = 0.0;
-    if (cf.vacuum_aware && nb.inflow)
+    if (with_pin && cf.vacuum_aware && nb.inflow)
         for (int e = 0; e < nb.nx * nb.ny; ++e)
             pin = fmax(pin, bm.spatial[(size_t)(nb.i0 + e / nb.ny) * cf.ny + (nb.j0 + e % nb.ny)] * ed);
     st->pin_max = pin;

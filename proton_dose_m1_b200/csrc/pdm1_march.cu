@@ -150,9 +150,27 @@ __global__ void __launch_bounds__(1024) tiles_kernel(const ConfigDev *cfp, const
 // ---------------------------------------------------------------------------
 // prologue: one CTA per step
 // ---------------------------------------------------------------------------
-constexpr int kEvalPerMat = 13;   // 5 stage energies + 8 Gauss points
+// Look-ups per material: S at 5 stage energies and 8 Gauss points, the transport and
+// the nuclear coefficient at the Gauss points.
+constexpr int kEvalS = 13, kEvalPerMat = kEvalS + 16;
 
-// One CTA per beam.
+// Optical depths over dE/3, dE/2, 2dE/3, dE
+__device__ __forceinline__ double depth_width(double dE, int d) {
+    return d == 0 ? dE / 3.0 : (d == 1 ? 0.5 * dE : (d == 2 ? 2.0 * dE / 3.0 : dE));
+}
+
+// Gauss point p of the depths (two per depth, energy.py:919-949)
+__device__ __forceinline__ double gauss_point(double E, double dE, int p) {
+    const double w = depth_width(dE, p >> 1);
+    const double mid = E - 0.5 * w, half = 0.5 * w, off = half / sqrt(3.0);
+    return p & 1 ? mid + off : mid - off;
+}
+
+// One CTA per beam, latency-bound: one thread decides the step, one thread takes each
+// table look-up (its loads issued together, table_dev), one thread each exponential with
+// the optical depth it needs.  Before, a thread took three look-ups in turn, one thread a
+// material's four depths, and each look-up a double logarithm (17.1 -> 14.0 us with cold
+// caches, 12x12x100 march 22.6 -> 20.9 ms).
 __global__ void __launch_bounds__(256) prologue_kernel(const ConfigDev *cfp, Coeffs *cos,
                                                        MarchState *sts, double *energies) {
     const ConfigDev &cf = *cfp;
@@ -161,172 +179,151 @@ __global__ void __launch_bounds__(256) prologue_kernel(const ConfigDev *cfp, Coe
     Coeffs *co = cos + b;
     MarchState *st = sts + b;
     if (cf.nbeams > 1) energies = nullptr;
-    __shared__ double sE, sdE, sEn;
-    __shared__ int sActive, sSlot;
-    __shared__ double eS[kMaxMat][kEvalPerMat], eTr[kMaxMat][8], eNu[kMaxMat][8];
-    __shared__ double gpt[8];
-    int t = threadIdx.x;
+    __shared__ double sE, sdE;
+    __shared__ int sActive;
+    __shared__ double eS[kMaxMat][kEvalS], eTr[kMaxMat][8], eNu[kMaxMat][8];
+    const int t = threadIdx.x;
     if (t == 0) {
         int active = 0, slot = -1;
-        double E = st->E, dE = 0.0, En = E;
-        if (!st->done && st->error == 0) {
-            if (!(E > cf.Emin) || (cf.step_limit >= 0 && st->step >= cf.step_limit)) {
+        const double E = st->E, forced = st->forced_dE;
+        const double inv = __longlong_as_double((long long)st->inv_bits);
+        const int done = st->done, step0 = st->step, ti = st->ti, taken = st->taken;
+        const double cells = (double)st->dom.nx * st->dom.ny * st->dom.nz;
+        const int ntiles = st->dom.ntiles;
+        int error = st->error;
+        double dE = 0.0, En = E;
+        if (!done && error == 0) {
+            if (!(E > cf.Emin) || (cf.step_limit >= 0 && step0 >= cf.step_limit)) {
                 st->done = 1;
-            } else if (st->step >= cf.max_steps) {
-                st->error |= ERR_DEV_MAXSTEPS;
+            } else if (step0 >= cf.max_steps) {
+                error |= ERR_DEV_MAXSTEPS;
                 st->done = 1;
             } else {
-                if (st->forced_dE > 0.0) {
-                    dE = st->forced_dE;
+                if (forced > 0.0) {
+                    dE = forced;
                 } else if (cf.schedule) {
                     // a prescribed energy schedule (another run's steps): the
                     // next energy is taken as given, past its end down to Emin
-                    dE = st->step + 1 < cf.n_schedule ? E - cf.schedule[st->step + 1] : E - cf.Emin;
+                    dE = step0 + 1 < cf.n_schedule ? E - cf.schedule[step0 + 1] : E - cf.Emin;
                 } else {
-                    double inv = __longlong_as_double((long long)st->inv_bits);
                     dE = cf.cfl / inv;
                     dE = cf.max_dE < dE ? cf.max_dE : dE;
-                    if (st->ti < cf.n_targets) {
-                        double tg = cf.targets[st->ti];
+                    if (ti < cf.n_targets) {
+                        double tg = cf.targets[ti];
                         if (E > tg && tg >= E - dE) dE = E - tg;
                     }
                     if (E - cf.Emin < dE) dE = E - cf.Emin;
                 }
                 if (!(dE > 0.0) || !isfinite(dE)) {
-                    st->error |= ERR_DEV_NONFINITE;
+                    error |= ERR_DEV_NONFINITE;
                     st->done = 1;
                 } else {
                     active = 1;
                     En = E - dE;
-                    if (cf.schedule && st->forced_dE <= 0.0 && st->step + 1 < cf.n_schedule)
-                        En = cf.schedule[st->step + 1];
-                    int step = st->step + 1;
+                    if (cf.schedule && forced <= 0.0 && step0 + 1 < cf.n_schedule) En = cf.schedule[step0 + 1];
+                    const int step = step0 + 1;
                     if (energies) energies[step] = En;
-                    if (st->ti < cf.n_targets && fabs(En - cf.targets[st->ti]) <= 1e-12) {
-                        slot = st->taken;
-                        st->taken += 1;
-                        st->ti += 1;
+                    if (ti < cf.n_targets && fabs(En - cf.targets[ti]) <= 1e-12) {
+                        slot = taken;
+                        st->taken = taken + 1;
+                        st->ti = ti + 1;
                     }
                     st->step = step;
                     st->E = En;
-                    const double cells = (double)st->dom.nx * st->dom.ny * st->dom.nz;
                     st->cell_steps += cells;
                     st->max_cells = fmax(st->max_cells, cells);
                     st->inv_bits = 0ull;
-                    if (st->forced_dE > 0.0) st->done = 1;
+                    if (forced > 0.0) st->done = 1;
                 }
             }
+            if (error) st->error = error;
         }
-        sE = E; sdE = dE; sEn = En; sActive = active; sSlot = slot;
+        sE = E; sdE = dE; sActive = active;
         co->E = E; co->dE = dE; co->E_next = En; co->active = active; co->snap_slot = slot;
         if (cf.nbeams == 1) {
             cf.tile_off[0] = 0;
-            cf.tile_off[1] = active ? st->dom.ntiles : 0;
+            cf.tile_off[1] = active ? ntiles : 0;
             cf.summary->active = active;
-            cf.summary->error = st->error;
+            cf.summary->error = error;
         }
     }
     __syncthreads();
     if (!sActive) return;
     const double E = sE, dE = sdE;
-    // Gauss points for the depths over dE/3, dE/2, 2dE/3, dE (energy.py:919-949)
-    if (t < 4) {
-        const double width[4] = {dE / 3.0, 0.5 * dE, 2.0 * dE / 3.0, dE};
-        double w = width[t];
-        double mid = E - 0.5 * w;
-        double half = 0.5 * w;
-        double off = half / sqrt(3.0);
-        gpt[2 * t] = mid - off;
-        gpt[2 * t + 1] = mid + off;
-    }
-    __syncthreads();
-    int nm = cf.nm;
-    if (t < nm * kEvalPerMat) {
-        int m = t / kEvalPerMat, q = t % kEvalPerMat;
+    const int nm = cf.nm;
+    for (int w = t; w < nm * kEvalPerMat; w += 256) {
+        const int m = w / kEvalPerMat, q = w % kEvalPerMat;
         const MatDev &mat = cf.mats[m];
         bool ok = true;
-        double e;
-        if (q < 5) {
-            const double stage_e[5] = {E, E - dE / 3.0, E - 2.0 * dE / 3.0, E - dE, E - 0.5 * dE};
-            e = stage_e[q];
+        if (q < kEvalS) {
+            const double e = q == 0 ? E : (q == 1 ? E - dE / 3.0 : (q == 2 ? E - 2.0 * dE / 3.0 : (q == 3 ? E - dE :
+                             (q == 4 ? E - 0.5 * dE : gauss_point(E, dE, q - 5)))));
+            double s = 1.0;
+            ok = stopping_power_dev(mat, e, s);
+            eS[m][q] = s;
         } else {
-            e = gpt[q - 5];
+            const int p = (q - kEvalS) & 7;
+            const double e = gauss_point(E, dE, p);
             double v = 0.0;
-            ok &= transport_dev(cf, mat, e, v);
-            eTr[m][q - 5] = v;
-            v = 0.0;
-            if (cf.nuclear) ok &= nuclear_dev(cf, mat, e, v);
-            eNu[m][q - 5] = v;
+            if (q < kEvalS + 8) {
+                ok = transport_dev(cf, mat, e, v);
+                eTr[m][p] = v;
+            } else {
+                if (cf.nuclear) ok = nuclear_dev(cf, mat, e, v);
+                eNu[m][p] = v;
+            }
         }
-        double s = 1.0;
-        ok &= stopping_power_dev(mat, e, s);
-        eS[m][q] = s;
         if (!ok) atomicOr(&st->error, ERR_DEV_RANGE);
-    } else if (t >= 224 && t < 229) {
-        int q = t - 224;
-        const double ed_e[5] = {E, E - dE / 3.0, E - 2.0 * dE / 3.0, E - dE, E - dE};
-        double v = energy_density(bm, ed_e[q]);
-        if (q < 4) co->ed[q] = v; else co->ed_next = v;
     }
     __syncthreads();
-    __shared__ double sTs[kMaxMat][4], sTn[kMaxMat][4];
     if (t < nm) {
-        int m = t;
+        const int m = t;
         co->S0[m] = eS[m][0];
         co->S1[m] = eS[m][3];
         co->S2[m] = eS[m][4];
-        co->Sb[0][m] = eS[m][0];
-        co->Sb[1][m] = eS[m][1];
-        co->Sb[2][m] = eS[m][2];
-        co->Sb[3][m] = eS[m][3];
-        // optical depths, physics/scattering.py:267-306 and nuclear.py:202-233
-        // depth index: 0 -> dE/3, 1 -> dE/2, 2 -> 2dE/3, 3 -> dE
-        const double width[4] = {dE / 3.0, 0.5 * dE, 2.0 * dE / 3.0, dE};
-        for (int d = 0; d < 4; ++d) {
-            double half = 0.5 * width[d];
-            double ts = 0.0, tn = 0.0;
-            if (cf.scattering != PDM1_SCATTERING_OFF)
-                ts = half * (eTr[m][2 * d] / eS[m][5 + 2 * d] + eTr[m][2 * d + 1] / eS[m][6 + 2 * d]);
-            if (cf.nuclear)
-                tn = half * (eNu[m][2 * d] / eS[m][5 + 2 * d] + eNu[m][2 * d + 1] / eS[m][6 + 2 * d]);
-            sTs[m][d] = ts;
-            sTn[m][d] = tn;
-        }
+        for (int q = 0; q < 4; ++q) co->Sb[q][m] = eS[m][q];
         co->fip[0][m] = 1.0;
         co->fic[0][m] = 1.0;
     }
-    __syncthreads();
-    // the 16 exponentials per material, one thread each (energy.py:273-310,
-    // 1168-1191): integrating factors C(tau) and C(tau)^-1 over dE and dE/2,
-    // the inverse factors of the inflow trace at dE/3, 2dE/3, dE, and the
-    // Strang half-step factors
-    if (t < nm * 16) {
-        const int m = t / 16, f = t % 16;
-        double ts = 0.0, tn = 0.0, out = 1.0;
+    // the exponentials: 16 per material (energy.py:273-310, 1168-1191): integrating
+    // factors C(tau) and C(tau)^-1 over dE and dE/2, the inverse factors of the inflow
+    // trace at dE/3, 2dE/3, dE, and the Strang half-step factors; then the spectrum at
+    // the stage energies and at the next one
+    for (int w = t; w < nm * 16 + 5; w += 256) {
+        if (w >= nm * 16) {
+            const int q = w - nm * 16;
+            const double v = energy_density(bm, q == 0 ? E : (q == 1 ? E - dE / 3.0 : (q == 2 ? E - 2.0 * dE / 3.0 : E - dE)));
+            if (q < 4) co->ed[q] = v;
+            else co->ed_next = v;
+            continue;
+        }
+        // factor f: depth index, inverse, of J (transport and nuclear) or of phi (nuclear)
+        const int m = w / 16, f = w % 16;
+        const int d = f < 4 ? 3 : (f < 8 ? 1 : (f < 10 ? 0 : (f < 12 ? 2 : 3)));
+        const bool inv = f < 8 ? (f & 2) != 0 : f < 14, cur = (f & 1) != 0;
+        // optical depths, physics/scattering.py:267-306 and nuclear.py:202-233
+        const double half = 0.5 * depth_width(dE, d);
+        double ts = 0.0, tn = 0.0;
+        if (cf.scattering != PDM1_SCATTERING_OFF)
+            ts = half * (eTr[m][2 * d] / eS[m][5 + 2 * d] + eTr[m][2 * d + 1] / eS[m][6 + 2 * d]);
+        if (cf.nuclear)
+            tn = half * (eNu[m][2 * d] / eS[m][5 + 2 * d] + eNu[m][2 * d + 1] / eS[m][6 + 2 * d]);
         if (f < 14) {
-            // which depth, and which factor of source_factor()
-            const int depth[14] = {3, 3, 3, 3, 1, 1, 1, 1, 0, 0, 2, 2, 3, 3};
-            const bool inv[14] = {false, false, true, true, false, false, true, true, true, true, true, true, true, true};
-            const bool cur[14] = {false, true, false, true, false, true, false, true, false, true, false, true, false, true};
-            if (cf.use_if) {
-                ts = sTs[m][depth[f]];
-                tn = sTn[m][depth[f]];
-            }
-            double sign = inv[f] ? 1.0 : -1.0;
-            double a = tn < kExpClamp ? tn : kExpClamp;
-            double tsum = tn + ts;
-            double b = tsum < kExpClamp ? tsum : kExpClamp;
-            out = dd_exp(sign * (cur[f] ? b : a));
-            double *dst[14] = {&co->c1p[m], &co->c1c[m], &co->c1ip[m], &co->c1ic[m],
-                               &co->c2p[m], &co->c2c[m], &co->c2ip[m], &co->c2ic[m],
-                               &co->fip[1][m], &co->fic[1][m], &co->fip[2][m], &co->fic[2][m],
-                               &co->fip[3][m], &co->fic[3][m]};
-            *dst[f] = out;
+            if (!cf.use_if) ts = tn = 0.0;
+            const double sign = inv ? 1.0 : -1.0;
+            const double a = tn < kExpClamp ? tn : kExpClamp;
+            const double tsum = tn + ts;
+            const double c = tsum < kExpClamp ? tsum : kExpClamp;
+            const double out = dd_exp(sign * (cur ? c : a));
+            double *dst = f < 2 ? (cur ? co->c1c : co->c1p) : (f < 4 ? (cur ? co->c1ic : co->c1ip) :
+                          (f < 6 ? (cur ? co->c2c : co->c2p) : (f < 8 ? (cur ? co->c2ic : co->c2ip) :
+                          (cur ? co->fic[(f - 6) >> 1] : co->fip[(f - 6) >> 1]))));
+            dst[m] = out;
         } else if (f == 14) {
-            double th = 0.5 * sTn[m][3];
+            double th = 0.5 * tn;
             co->hn[m] = (cf.strang && cf.nuclear) ? dd_exp(-(th < kExpClamp ? th : kExpClamp)) : 1.0;
         } else {
-            double th = 0.5 * sTs[m][3];
+            double th = 0.5 * ts;
             co->hs[m] = (cf.strang && cf.scattering != PDM1_SCATTERING_OFF)
                             ? dd_exp(-(th < kExpClamp ? th : kExpClamp)) : 1.0;
         }
@@ -494,14 +491,11 @@ __global__ void __launch_bounds__(256) box_kernel(const ConfigDev *cfp, Coeffs *
     Coeffs *co = cos + b;
     MarchState *st = sts + b;
     unsigned long long *slab = beam_slab(cf, b);
-    __shared__ double red[512];   // significant_box_cta: two reductions
+    __shared__ double red[16];   // significant_box_cta
     __shared__ double s_ed, s_scale;
     __shared__ int s_lo[3], s_hi[3];
-    __shared__ int s_done;
     const int t = threadIdx.x;
-    if (t == 0) s_done = st->done || st->error;
-    __syncthreads();
-    if (s_done) return;
+    if (__syncthreads_or(t == 0 && (st->done || st->error))) return;
     const DomainDev d = st->dom;
     const double E = st->E;
     // init_kernel and prologue_kernel leave S1 = S(E_next) and ed_next =
@@ -545,7 +539,23 @@ __global__ void __launch_bounds__(256) box_kernel(const ConfigDev *cfp, Coeffs *
             int bk0 = ak0 - g > 0 ? ak0 - g : 0, bk1 = ak1 + g < cf.nz ? ak1 + g : cf.nz;
             nb = make_domain(bi0, bj0, bk0, bi1 - bi0, bj1 - bj0, bk1 - bk0, bk0 == 0, cf.tile);
         }
-        switch_box(cf, bm, co, st, b, nb, ed);
+        switch_box(cf, bm, co, st, b, nb, ed, false);
+    }
+    if (cf.vacuum_aware && !cf.learned) {   // the largest inflow over the new box's entrance
+        __syncthreads();
+        const DomainDev nb = st->dom;
+        double pin = 0.0;
+        if (nb.inflow)
+            for (int i = t >> 5; i < nb.nx; i += 8)
+                for (int j = t & 31; j < nb.ny; j += 32)
+                    pin = fmax(pin, bm.spatial[(size_t)(nb.i0 + i) * cf.ny + (nb.j0 + j)] * ed);
+        for (int w = 16; w > 0; w >>= 1) pin = fmax(pin, __shfl_xor_sync(0xffffffffu, pin, w));
+        if ((t & 31) == 0) red[t >> 5] = pin;
+        __syncthreads();
+        if (t == 0) {
+            for (int w = 0; w < 8; ++w) pin = fmax(pin, red[w]);
+            st->pin_max = pin;
+        }
     }
 }
 
@@ -739,10 +749,10 @@ std::vector<double> host_pchip_slopes(const double *E, const double *v, int n) {
 struct pdm1_plan {
     pdm1_problem p{};
     ConfigDev cf{};
+    ConfigDev *d_cf = nullptr;
     int nbeams = 1;
     bool field = false;              // created by pdm1_field_plan_create
     size_t cap = 0;
-    ConfigDev *d_cf = nullptr;
     Coeffs *d_co = nullptr;         // nbeams
     MarchState *d_st = nullptr;     // nbeams
     MarchState *h_st = nullptr;     // pinned, nbeams
@@ -926,6 +936,7 @@ void launch_stage(const pdm1_plan *pl, int mode, int grid, const StageArgs &a, c
     switch (pl->cf.tile_id) {
     case 1: launch_stage64<Tile1>(mode, grid, a, stream); break;
     case 2: launch_stage64<Tile2>(mode, grid, a, stream); break;
+    case kSmallTileId: launch_stage64<SmallTile>(mode, grid, a, stream); break;
     default: launch_stage64<Tile0>(mode, grid, a, stream); break;
     }
 }
@@ -1012,6 +1023,7 @@ int set_smem_attributes() {
     CUDA_TRY(set_attributes64<Tile0>());
     CUDA_TRY(set_attributes64<Tile1>());
     CUDA_TRY(set_attributes64<Tile2>());
+    CUDA_TRY(set_attributes64<SmallTile>());
     CUDA_TRY((cudaError_t)stage_fp32_set_attributes());
     done = true;
     return PDM1_OK;
@@ -1090,10 +1102,17 @@ void destroy_plan(pdm1_plan *pl) {
 // 80 registers: -4 % stage time on field256).
 int stage_slots(const pdm1_problem &p, int sms) { return (p.precision == PDM1_FP32_FP64 ? 4 : 2) * sms; }
 
+// The tile shape of a plan: `id` of kTiles, or SmallTile where the grids of all
+// beams fit one wave of it.
+void choose_tile(const pdm1_problem &p, int id, int nbeams, int sms, TileDims &t, int &tile_id) {
+    const size_t n = (size_t)make_domain(0, 0, 0, p.nx, p.ny, p.nz, 1, kSmallTile).ntiles * nbeams;
+    const bool small = n <= (size_t)stage_slots(p, sms);
+    t = small ? kSmallTile : kTiles[id];
+    tile_id = small ? kSmallTileId : id;
+}
+
 int stage_grid(const pdm1_problem &p, TileDims t, int nbeams, int sms) {
-    // a moving box may take small tiles where the full grid does not
-    const size_t tiles = std::max<size_t>(make_domain(0, 0, 0, p.nx, p.ny, p.nz, 1, t).ntiles,
-                                          p.moving_active_domain ? t.small : 0) * nbeams;
+    const size_t tiles = (size_t)make_domain(0, 0, 0, p.nx, p.ny, p.nz, 1, t).ntiles * nbeams;
     return (int)std::max<size_t>(1, std::min<size_t>(tiles, stage_slots(p, sms)));
 }
 
@@ -1121,8 +1140,7 @@ int create_plan(const pdm1_problem *problem, const pdm1_beam *beams, int nbeams,
         if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         pl->sms = sms;
     }
-    cf.tile = with_small(kTiles[0], stage_slots(p, pl->sms), nbeams);
-    cf.tile_id = 0;
+    choose_tile(p, 0, nbeams, pl->sms, cf.tile, cf.tile_id);
     cf.dx = p.dx; cf.dy = p.dy; cf.dz = p.dz;
     cf.inv_dx = 1.0 / p.dx; cf.inv_dy = 1.0 / p.dy; cf.inv_dz = 1.0 / p.dz;
     cf.spacing_near = near_spacing(p.dx) && near_spacing(p.dy) && near_spacing(p.dz);
@@ -1147,7 +1165,7 @@ int create_plan(const pdm1_problem *problem, const pdm1_beam *beams, int nbeams,
         cf.mats[m].sp = add_table(blob, fix, mt.stopping_power);
         cf.mats[m].tr = add_table(blob, fix, mt.transport);
         cf.mats[m].nuc = add_table(blob, fix, mt.nuclear);
-        cf.mats[m].density = mt.density;
+        cf.mats[m].density = cf.density[m] = mt.density;
         cf.mats[m].X0 = mt.radiation_length;
         const pdm1_table *tabs[3] = {&mt.stopping_power, &mt.transport, &mt.nuclear};
         for (int q = 0; q < 3; ++q) {
@@ -1467,9 +1485,8 @@ int pdm1_tile_shape(int tile_id, int *tx, int *ty, int *tz) {
 int pdm1_plan_set_tile(pdm1_plan *pl, int tile_id) {
     if (!pl) return set_error(PDM1_ERR_ARGUMENT, "plan is NULL");
     if (tile_id < 0 || tile_id >= kNumTiles) return set_error(PDM1_ERR_ARGUMENT, "unknown tile shape");
-    const TileDims t = with_small(kTiles[tile_id], stage_slots(pl->p, pl->sms), pl->nbeams);
-    pl->cf.tile = t;
-    pl->cf.tile_id = tile_id;
+    choose_tile(pl->p, tile_id, pl->nbeams, pl->sms, pl->cf.tile, pl->cf.tile_id);
+    const TileDims t = pl->cf.tile;
     pl->cf.grid_ctas = stage_grid(pl->p, t, pl->nbeams, pl->sms);
     for (BeamDev &bd : pl->h_beams) {
         const DomainDev &o = bd.init_box;
@@ -1899,7 +1916,7 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
     cf.nx = p.nx; cf.ny = p.ny; cf.nz = p.nz;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cf.tile = with_small(kTiles[0], stage_slots(p, sms), 1);
+    cf.tile = kTiles[0];
     cf.tile_id = 0;
     cf.dx = p.dx; cf.dy = p.dy; cf.dz = p.dz;
     cf.inv_dx = 1.0 / p.dx; cf.inv_dy = 1.0 / p.dy; cf.inv_dz = 1.0 / p.dz;
@@ -1952,7 +1969,7 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
             CUDA_TRY(cudaMemcpyAsync(dE_ + t.n_nodes, t.value, t.n_nodes * sizeof(double), cudaMemcpyHostToDevice, stream));
             pchip_slopes_kernel<<<(t.n_nodes + 255) / 256, 256, 0, stream>>>(dE_, dE_ + t.n_nodes, dE_ + 2 * t.n_nodes, t.n_nodes);
         }
-        cf.mats[m].density = mt.density;
+        cf.mats[m].density = cf.density[m] = mt.density;
         cf.mats[m].X0 = mt.radiation_length;
     }
     CUDA_TRY(cudaMemcpyAsync(base + o_ids, p.ids, N * sizeof(int32_t), cudaMemcpyHostToDevice, stream));

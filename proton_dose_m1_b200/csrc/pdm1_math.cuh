@@ -47,14 +47,6 @@ PDM1_HD dd dd_mul(dd a, dd b) {
     return dd_quick(p, e);
 }
 
-PDM1_HD dd dd_div_d(double a, double b) {
-    double q1 = a / b;
-    double p = q1 * b;
-    double e = fma(q1, b, -p);
-    double rem = (a - p) - e;
-    return dd_quick(q1, rem / b);
-}
-
 PDM1_HD double dd_exp(double x) {
     if (x != x) return x;
     if (x > 709.782712893384) return INFINITY;
@@ -69,9 +61,17 @@ PDM1_HD double dd_exp(double x) {
     dd r = dd_quick(s, t);
     r.hi *= 0x1p-10;
     r.lo *= 0x1p-10;
-    const double fact[10] = {1.0, 1.0, 2.0, 6.0, 24.0, 120.0, 720.0, 5040.0, 40320.0, 362880.0};
-    dd acc = dd_div_d(1.0, fact[9]);
-    for (int n = 8; n >= 0; --n) acc = dd_add(dd_mul(acc, r), dd_div_d(1.0, fact[n]));
+    // 1/n! as double-doubles
+    constexpr double ch[10] = {0x1.0000000000000p+0, 0x1.0000000000000p+0, 0x1.0000000000000p-1, 0x1.5555555555555p-3,
+                               0x1.5555555555555p-5, 0x1.1111111111111p-7, 0x1.6c16c16c16c17p-10, 0x1.a01a01a01a01ap-13,
+                               0x1.a01a01a01a01ap-16, 0x1.71de3a556c734p-19};
+    constexpr double cl[10] = {0.0, 0.0, 0.0, 0x1.5555555555555p-57,
+                               0x1.5555555555555p-59, 0x1.1111111111111p-63, -0x1.f49f49f49f49fp-65, 0x1.a01a01a01a01ap-73,
+                               0x1.a01a01a01a01ap-76, -0x1.c154f8ddc6c00p-73};
+    dd acc = {ch[9], cl[9]};
+#pragma unroll
+    for (int n = 8; n >= 0; --n) acc = dd_add(dd_mul(acc, r), dd{ch[n], cl[n]});
+#pragma unroll
     for (int q = 0; q < 10; ++q) acc = dd_mul(acc, acc);
     return ldexp(acc.hi + acc.lo, (int)k);
 }
@@ -627,11 +627,18 @@ struct TableView {
     double log_e0, inv_log_step;   // inv_log_step == 0: no log guess
 };
 
+// First guess of the interval from the log spacing; the comparisons that follow
+// make it exact, so a single-precision logarithm (off by less than a hundredth of
+// an interval on 6000 nodes over six decades) serves as well as a double one.
+PDM1_HD int interval_guess(const TableView &t, double x) {
+    const float g = (logf((float)x) - (float)t.log_e0) * (float)t.inv_log_step;
+    return g < 0.0f ? 0 : (g > (float)(t.n - 1) ? t.n - 1 : (int)g);
+}
+
 PDM1_HD int search_right(const TableView &t, double x) {
     int g;
     if (t.inv_log_step > 0.0 && x > 0.0) {
-        double gf = (log(x) - t.log_e0) * t.inv_log_step;
-        g = gf < 0.0 ? 0 : (gf > (double)(t.n - 1) ? t.n - 1 : (int)gf);
+        g = interval_guess(t, x);
     } else {
         int lo = 0, hi = t.n;
         while (lo < hi) {
@@ -645,21 +652,38 @@ PDM1_HD int search_right(const TableView &t, double x) {
     return g;
 }
 
-PDM1_HD double pchip_eval(const TableView &t, double x) {
-    int n = t.n;
-    if (x >= t.E[n - 1]) return t.v[n - 1];
-    int i = search_right(t, x);
-    if (i < 0) i = 0;
-    if (i > n - 2) i = n - 2;
-    double h = t.E[i + 1] - t.E[i];
-    double s = (x - t.E[i]) / h;
+// Cubic Hermite on [e0, e1]
+PDM1_HD double pchip_interval(double e0, double e1, double v0, double v1, double s0, double s1, double x) {
+    double h = e1 - e0;
+    double s = (x - e0) / h;
     double s2 = s * s;
     double s3 = s2 * s;
     double h00 = 2.0 * s3 - 3.0 * s2 + 1.0;
     double h10 = s3 - 2.0 * s2 + s;
     double h01 = -2.0 * s3 + 3.0 * s2;
     double h11 = s3 - s2;
-    return h00 * t.v[i] + h10 * h * t.slope[i] + h01 * t.v[i + 1] + h11 * h * t.slope[i + 1];
+    return h00 * v0 + h10 * h * s0 + h01 * v1 + h11 * h * s1;
+}
+
+PDM1_HD double pchip_eval(const TableView &t, double x) {
+    int n = t.n;
+    if (x >= t.E[n - 1]) return t.v[n - 1];
+    int i = search_right(t, x);
+    if (i < 0) i = 0;
+    if (i > n - 2) i = n - 2;
+    return pchip_interval(t.E[i], t.E[i + 1], t.v[i], t.v[i + 1], t.slope[i], t.slope[i + 1], x);
+}
+
+// numpy.interp on [e0, e1) (its value at a node, its repair of a NaN)
+PDM1_HD double linear_interval(double e0, double e1, double v0, double v1, double x) {
+    if (e0 == x) return v0;
+    double slope = (v1 - v0) / (e1 - e0);
+    double r = slope * (x - e0) + v0;
+    if (r != r) {
+        r = slope * (x - e1) + v1;
+        if (r != r && v0 == v1) r = v0;
+    }
+    return r;
 }
 
 PDM1_HD double linear_eval(const TableView &t, double x) {
@@ -668,19 +692,11 @@ PDM1_HD double linear_eval(const TableView &t, double x) {
     if (x > t.E[n - 1]) return t.v[n - 1];
     int j = search_right(t, x);
     if (j >= n - 1) return t.v[n - 1];
-    if (t.E[j] == x) return t.v[j];
-    double slope = (t.v[j + 1] - t.v[j]) / (t.E[j + 1] - t.E[j]);
-    double r = slope * (x - t.E[j]) + t.v[j];
-    if (r != r) {
-        r = slope * (x - t.E[j + 1]) + t.v[j + 1];
-        if (r != r && t.v[j] == t.v[j + 1]) r = t.v[j];
-    }
-    return r;
+    return linear_interval(t.E[j], t.E[j + 1], t.v[j], t.v[j + 1], x);
 }
 
 // numpy.isclose(a, b) with rtol 1e-5, atol 1e-8; clip of stopping_power.py:151-170
-PDM1_HD bool clip_energy(const TableView &t, double &x) {
-    double lo = t.E[0], hi = t.E[t.n - 1];
+PDM1_HD bool clip_energy(double lo, double hi, double &x) {
     bool close_lo = fabs(x - lo) <= 1e-8 + 1e-5 * fabs(lo);
     bool close_hi = fabs(x - hi) <= 1e-8 + 1e-5 * fabs(hi);
     if ((x < lo && !close_lo) || (x > hi && !close_hi)) return false;

@@ -535,7 +535,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
                 // a non-finite state ends the march with PDM1_ERR_NONFINITE
                 if (!finite) atomicOr(&stb.error, ERR_DEV_NONFINITE);
                 if (a.edep) a.edep[o] = ed;
-                else atomicAdd(&a.dose[go], ed * kMevToJoule / cf.mats[m].density);
+                else atomicAdd(&a.dose[go], ed * kMevToJoule / cf.density[m]);
                 if (MODE == MODE_C) {
                     if (co.snap_slot >= 0 && a.snap) {
                         const size_t NG = (size_t)cf.nx * cf.ny * cf.nz;
@@ -566,15 +566,6 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
     }
 }
 
-// The small tile in a function of its own: inlined beside the other shape, the
-// two share registers and spill.
-template <typename T, int MODE, bool LEARN>
-__device__ __noinline__ double small_stage_tile(const StageArgs &a, int b, int tile, unsigned bar_phase, double cta_inv) {
-    const DomainDev d = a.st[b].dom;
-    stage_tile<T, MODE, SmallTile, LEARN>(a, *a.cf, d, b, tile, bar_phase, cta_inv);
-    return cta_inv;
-}
-
 // LEARN (stage C of a plan with a learned box): the tile's fluence moments of
 // the new state are accumulated for the next step's proposer.
 template <typename T, int MODE, class Tl, bool LEARN = false>
@@ -597,8 +588,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == sizeof(double) ? 2 : 4) stage
         const int b = (MODE == MODE_RHS || cf.nbeams == 1) ? 0 : beam_of_tile(cf.tile_off, cf.nbeams, gt);
         const int tile = MODE == MODE_RHS ? gt : gt - cf.tile_off[b];
         const DomainDev d = a.st[b].dom;
-        if (d.small) cta_inv = small_stage_tile<T, MODE, LEARN>(a, b, tile, bar_phase, cta_inv);
-        else stage_tile<T, MODE, Tl, LEARN>(a, cf, d, b, tile, bar_phase, cta_inv);
+        stage_tile<T, MODE, Tl, LEARN>(a, cf, d, b, tile, bar_phase, cta_inv);
         bar_phase ^= 1u;
         __syncthreads();   // shared memory is reused by the next tile
     }

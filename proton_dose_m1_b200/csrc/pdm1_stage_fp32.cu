@@ -5,7 +5,7 @@
 // projection near |J|/phi -> 1, the CFL bound and the dose accumulation stay
 // in double (pdm1_stage.cuh).  Compiled with --use_fast_math: approximate
 // division and square root in the float stencil, FMA contraction throughout.
-// One instantiation per tile shape of kTiles.
+// One instantiation per tile shape.
 #include "pdm1_stage.cuh"
 
 namespace pdm1 {
@@ -45,6 +45,7 @@ int stage_fp32_set_attributes() {
     cudaError_t e = set_attributes<Tile0>();
     if (e == cudaSuccess) e = set_attributes<Tile1>();
     if (e == cudaSuccess) e = set_attributes<Tile2>();
+    if (e == cudaSuccess) e = set_attributes<SmallTile>();
     return (int)e;
 }
 
@@ -52,6 +53,7 @@ void launch_stage_fp32(int mode, int tile_id, int grid, const StageArgs &a, cuda
     switch (tile_id) {
     case 1: launch<Tile1>(mode, grid, a, stream); break;
     case 2: launch<Tile2>(mode, grid, a, stream); break;
+    case kSmallTileId: launch<SmallTile>(mode, grid, a, stream); break;
     default: launch<Tile0>(mode, grid, a, stream); break;
     }
 }
