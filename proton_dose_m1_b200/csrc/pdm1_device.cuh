@@ -13,6 +13,7 @@
 namespace pdm1 {
 
 constexpr int kMaxMat = 16;
+constexpr int kTileCounters = 3;   // behind the tile offsets: one per stage
 
 // Learned moving box: proposer network 16 -> 64 -> 64 -> 6 (ReLU).
 constexpr int kFeat = 16, kHid = 64, kOut = 6, kOutPad = 8;
@@ -98,7 +99,8 @@ struct ConfigDev {
     int nbeams;
     size_t cap;
     const BeamDev *beams;
-    int *tile_off;              // (nbeams + 1) prefix sums of the active beams' tiles
+    int *tile_off;              // (nbeams + 1) prefix sums of the active beams' tiles, then the
+                                // tiles handed out beyond the grid's first in stages A, B, C
     MarchSummary *summary;
     // moving active box
     int moving, vacuum_aware, guard;
@@ -240,9 +242,10 @@ constexpr int NT = 256;   // threads of a stage CTA
 
 // A tile shape: the tile's cells, its cross-shaped 3-cell WENO halo (no
 // corners: WENO reads along one axis at a time) and its faces.  Shared memory
-// holds three arms per component, each the core plus the halo along one axis
-// (the core stored three times), so every 6-point stencil is a strided run in
-// one arm.
+// holds, in float, three arms per component, each the core plus the halo along
+// one axis (the core stored three times), so every 6-point stencil is a strided
+// run in one arm; in double one copy of every cell (the x arm, then the y and z
+// halos): a third less, so that three CTAs fit an SM.
 template <int X, int Y, int Z>
 struct Tile {
     static constexpr int CELLS = X * Y * Z;
@@ -257,7 +260,9 @@ struct Tile {
     static constexpr int AY = X * (Y + 6) * Z;
     static constexpr int AZ = X * Y * (Z + 6);
     template <typename T>
-    static constexpr size_t arm_bytes() { return sizeof(T) * 4 * (AX + AY + AZ + NF); }
+    static constexpr size_t arm_bytes() {
+        return sizeof(T) * 4 * ((sizeof(T) == sizeof(double) ? SX + SY + SZ : AX + AY + AZ) + NF);
+    }
 };
 
 // The tile shapes the stage kernels are built for, the autotuner's candidates.

@@ -140,6 +140,7 @@ __global__ void __launch_bounds__(1024) tiles_kernel(const ConfigDev *cfp, const
         if (t == blockDim.x - 1) carry += scan[t];
         __syncthreads();
     }
+    if (t < kTileCounters) cf.tile_off[cf.nbeams + 1 + t] = 0;
     if (t == 0) {
         cf.tile_off[0] = 0;
         cf.summary->active = n_active;
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(256) prologue_kernel(const ConfigDev *cfp, Coe
         if (cf.nbeams == 1) {
             cf.tile_off[0] = 0;
             cf.tile_off[1] = active ? ntiles : 0;
+            for (int q = 0; q < kTileCounters; ++q) cf.tile_off[2 + q] = 0;
             cf.summary->active = active;
             cf.summary->error = error;
         }
@@ -1203,7 +1205,7 @@ int create_plan(const pdm1_problem *problem, const pdm1_beam *beams, int nbeams,
     ALLOC(pl->d_st, B * sizeof(MarchState));
     ALLOC(pl->d_sum, sizeof(MarchSummary));
     ALLOC(pl->d_beams, B * sizeof(BeamDev));
-    ALLOC(pl->d_tile_off, (B + 1) * sizeof(int));
+    ALLOC(pl->d_tile_off, (B + 1 + kTileCounters) * sizeof(int));
     ALLOC(pl->d_ids, N * sizeof(int32_t));
     ALLOC(pl->d_spatial, B * NXY * sizeof(double));
     ALLOC(pl->d_targets, 64 * sizeof(double));
@@ -1325,7 +1327,7 @@ int march_impl(pdm1_plan *pl, double *U, double *dose, double *energies, int max
         CUDA_TRY(cudaMemsetAsync(snap_out, 0, tg.size() * 4 * N * sizeof(double), stream));
     CUDA_TRY(cudaMemsetAsync(pl->d_acc, 0, (size_t)B * kAcc * sizeof(double), stream));
     CUDA_TRY(cudaMemsetAsync(pl->d_plane, 0, (size_t)B * p.nz * sizeof(double), stream));
-    CUDA_TRY(cudaMemsetAsync(pl->d_tile_off, 0, (size_t)(B + 1) * sizeof(int), stream));
+    CUDA_TRY(cudaMemsetAsync(pl->d_tile_off, 0, (size_t)(B + 1 + kTileCounters) * sizeof(int), stream));
     if (!p.moving_active_domain)
         CUDA_TRY(cudaMemsetAsync(pl->d_slab, 0, (size_t)B * (p.nx + p.ny + p.nz) * sizeof(unsigned long long), stream));
     (void)cudaGetLastError();   // start from a clean launch-error state
@@ -1847,7 +1849,7 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
     const size_t o_co = off; off = align256(off + sizeof(Coeffs));
     const size_t o_st = off; off = align256(off + sizeof(MarchState));
     const size_t o_bm = off; off = align256(off + sizeof(BeamDev));
-    const size_t o_to = off; off = align256(off + 2 * sizeof(int));
+    const size_t o_to = off; off = align256(off + (2 + kTileCounters) * sizeof(int));
     const size_t o_sm = off; off = align256(off + sizeof(MarchSummary));
     size_t o_tab[kMaxMat][3];
     for (int m = 0; m < p.n_materials; ++m) {

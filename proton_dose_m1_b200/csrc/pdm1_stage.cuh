@@ -144,7 +144,7 @@ struct StageShared {
     double mom_part[NT / 32][ACC_MAX + 1];   // learned box: moments of the new state
     double mom_pl[kMaxTileZ];
     unsigned long long stage_bar;    // FP32 stages B and C: the tile's bulk copies
-    unsigned long long pad;
+    int next_tile[2];                // the CTA's next tile, by the parity of the tile it is on
 };
 static_assert(sizeof(StageShared) % 16 == 0, "the arms behind it are 16-byte aligned");
 
@@ -168,6 +168,10 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
     s.Y = s.X + 4 * AX;    // [c][i][j + 3][k]
     s.Z = s.Y + 4 * AY;    // [c][i][j][k + 3]
     s.F = s.Z + 4 * AZ;
+    // double: component c at s.X + c * kCells: [i + 3][j][k], the y halo [i][0..2 | 3..5][k]
+    // from kHaloY on, the z halo [i][j][0..2 | 3..5] from kHaloZ on
+    constexpr int kCells = SX + SY + SZ, kHaloY = SX, kHaloZ = SX + SY;
+    if constexpr (kNear) s.F = s.X + 4 * kCells;
     int tid = threadIdx.x;
     asm volatile("" : "+r"(tid));   // the indices that follow from it are formed per tile: hoisted, they spill
     const bool unit = cf.unit_speeds != 0;
@@ -236,12 +240,19 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         load_cell<MODE>(cf, co, d, src, i0 + ii - 3, j0 + j, k0 + k, u);
         const bool core = ii >= 3 && ii < TX + 3;
         const int ex = (ii * TY + j) * TZ + k;
+        if constexpr (kNear) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                out_of_range |= !weno_range(u[c]);
+                s.X[c * kCells + ex] = u[c];
+            }
+            continue;
+        }
         const int ey = ((ii - 3) * (TY + 6) + j + 3) * TZ + k;
         const int ez = ((ii - 3) * TY + j) * (TZ + 6) + k + 3;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const T v = T(u[c]);
-            if constexpr (kNear) out_of_range |= !weno_range(u[c]);
             arm_at(s.X, AX, c, ex) = v;
             if (core) {
                 arm_at(s.Y, AY, c, ey) = v;
@@ -257,8 +268,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         load_cell<MODE>(cf, co, d, src, i0 + i, gj, k0 + k, u);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            if constexpr (kNear) out_of_range |= !weno_range(u[c]);
-            arm_at(s.Y, AY, c, (i * (TY + 6) + aj) * TZ + k) = T(u[c]);
+            if constexpr (kNear) {
+                out_of_range |= !weno_range(u[c]);
+                s.X[c * kCells + kHaloY + e] = u[c];
+            } else {
+                arm_at(s.Y, AY, c, (i * (TY + 6) + aj) * TZ + k) = T(u[c]);
+            }
         }
     }
     for (int e = tid; e < SZ; e += NT) {
@@ -270,8 +285,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         load_cell<MODE>(cf, co, d, src, i0 + i, j0 + j, gk, u);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            if constexpr (kNear) out_of_range |= !weno_range(u[c]);
-            arm_at(s.Z, AZ, c, (i * TY + j) * (TZ + 6) + ak) = T(u[c]);
+            if constexpr (kNear) {
+                out_of_range |= !weno_range(u[c]);
+                s.X[c * kCells + kHaloZ + e] = u[c];
+            } else {
+                arm_at(s.Z, AZ, c, (i * TY + j) * (TZ + 6) + ak) = T(u[c]);
+            }
         }
     }
     }   // the double-precision source
@@ -286,7 +305,11 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
             if (li >= nx || lj >= ny) continue;
             T ui = T(boundary_value<MODE>(a, cf, bm, co, d, c, li, lj));
             const int ez = (i * TY + j) * (TZ + 6);
-            auto z = [&](int kk) -> T & { return arm_at(s.Z, AZ, c, ez + kk); };
+            auto z = [&](int kk) -> T & {   // cell k0 - 3 + kk
+                if constexpr (kNear)
+                    return s.X[c * kCells + (kk < 3 ? kHaloZ + (i * TY + j) * 6 + kk : ((i + 3) * TY + j) * TZ + kk - 3)];
+                else return arm_at(s.Z, AZ, c, ez + kk);
+            };
             T u0 = z(3), u1 = z(4), u2 = z(5), u3 = z(6);
             if (cf.spatial == PDM1_SPATIAL_WENO_Z) {   // quartic, boundary.py:247-320
                 z(2) = T(5.0) * ui - T(77.0 / 12.0) * u0 + T(43.0 / 12.0) * u1 - T(17.0 / 12.0) * u2 + T(0.25) * u3;
@@ -303,24 +326,53 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         if constexpr (kNear) ieee = __syncthreads_or(out_of_range) != 0;
         else __syncthreads();
     }
-    // ---- 3. every face of the tile: WENO-Z, projection, HLL ----
-    for (int f = tid; f < NF; f += NT) {
-        int axis, i, j, k;
-        if (f < NFX) {
-            axis = 0; k = f % TZ; j = (f / TZ) % TY; i = f / (TZ * TY);
-        } else if (f < NFX + NFY) {
-            int u = f - NFX;
-            axis = 1; k = u % TZ; j = (u / TZ) % (TY + 1); i = u / (TZ * (TY + 1));
+    // ---- 3. every face of the tile's cells inside the domain: WENO-Z, projection, HLL ----
+    // A ragged tile (the domain ends inside it) enumerates only those, in the same flux
+    // slots: on 45x51x187 the padding is 17 % of the cells.
+    const int vx = min(TX, nx - i0), vy = min(TY, ny - j0), vz = min(TZ, nz - k0);
+    const bool full = vx == TX && vy == TY && vz == TZ;
+    const int nfx = full ? NFX : (vx + 1) * vy * vz, nfy = full ? NFY : vx * (vy + 1) * vz;
+    const int nf = full ? NF : nfx + nfy + vx * vy * (vz + 1);
+    for (int f = tid; f < nf; f += NT) {
+        int axis, i, j, k, slot = f;
+        if (full) {
+            if (f < NFX) {
+                axis = 0; k = f % TZ; j = (f / TZ) % TY; i = f / (TZ * TY);
+            } else if (f < NFX + NFY) {
+                int u = f - NFX;
+                axis = 1; k = u % TZ; j = (u / TZ) % (TY + 1); i = u / (TZ * (TY + 1));
+            } else {
+                int u = f - NFX - NFY;
+                axis = 2; k = u % (TZ + 1); j = (u / (TZ + 1)) % TY; i = u / ((TZ + 1) * TY);
+            }
         } else {
-            int u = f - NFX - NFY;
-            axis = 2; k = u % (TZ + 1); j = (u / (TZ + 1)) % TY; i = u / ((TZ + 1) * TY);
+            axis = f < nfx ? 0 : (f < nfx + nfy ? 1 : 2);
+            const int u = f - (axis == 0 ? 0 : (axis == 1 ? nfx : nfx + nfy));
+            const int ez = axis == 2 ? vz + 1 : vz, ey = axis == 1 ? vy + 1 : vy;   // faces along z and y
+            const int row = u / ez;
+            k = u - row * ez;
+            i = row / ey;
+            j = row - i * ey;
+            slot = axis == 0 ? (i * TY + j) * TZ + k
+                             : (axis == 1 ? NFX + (i * (TY + 1) + j) * TZ + k : NFX + NFY + (i * TY + j) * (TZ + 1) + k);
         }
         T L[4], R[4];
         // the six cells along the axis, i - 3 .. i + 2 (face between i - 1 and i),
         // are arm indices i .. i + 5
-        T *arm;
-        int e0, stride, cs;
-        if (axis == 0) {
+        T *arm = s.X;
+        int e0 = 0, stride = 0, cs = kCells, off[6];
+        if constexpr (kNear) {
+            const int pos = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 1 ? TY : TZ;
+            const int st = axis == 0 ? TY * TZ : (axis == 1 ? TZ : 1);
+            const int c0 = axis == 0 ? j * TZ + k : (axis == 1 ? (i + 3) * TY * TZ + k : ((i + 3) * TY + j) * TZ);
+            const int h0 = axis == 1 ? kHaloY + i * 6 * TZ + k : kHaloZ + (i * TY + j) * 6;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const int p = pos - 3 + q;
+                const bool core = axis == 0 || (p >= 0 && p < n);
+                off[q] = core ? c0 + (axis == 0 ? p + 3 : p) * st : h0 + (p < 0 ? p + 3 : p - n + 3) * st;
+            }
+        } else if (axis == 0) {
             arm = s.X; e0 = (i * TY + j) * TZ + k; stride = TY * TZ; cs = AX;
         } else if (axis == 1) {
             arm = s.Y; e0 = (i * (TY + 6) + j) * TZ + k; stride = TZ; cs = AY;
@@ -346,25 +398,38 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
                 r = weno_left_f32x2(w23[5], w23[4], w23[3], w23[2], w23[1]);
                 L[2] = l.x; L[3] = l.y; R[2] = r.x; R[3] = r.y;
             } else {
-                const T *base = arm + e0;
+                if (!ieee) {
+                    // no branch between the components: their chains interleave
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    T w[6];
+                    for (int c = 0; c < 4; ++c) {
+                        T w[6];
 #pragma unroll
-                    for (int q = 0; q < 6; ++q) w[q] = base[c * cs + q * stride];
-                    if (ieee) {
-                        L[c] = weno_left_ieee(w[0], w[1], w[2], w[3], w[4]);
-                        R[c] = weno_left_ieee(w[5], w[4], w[3], w[2], w[1]);
-                    } else {
+                        for (int q = 0; q < 6; ++q) w[q] = arm[c * cs + off[q]];
                         weno_pair(w, L[c], R[c]);
+                    }
+                } else {
+                    for (int c = 0; c < 4; ++c) {
+                        T w[6];
+#pragma unroll
+                        for (int q = 0; q < 6; ++q) w[q] = arm[c * cs + off[q]];
+                        const T l = weno_left_ieee(w[0], w[1], w[2], w[3], w[4]);
+                        const T r = weno_left_ieee(w[5], w[4], w[3], w[2], w[1]);
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (q == c) { L[q] = l; R[q] = r; }
                     }
                 }
             }
         } else {
             // the narrower stencils read cells i-2 .. i+1 (arm indices i+1 .. i+4)
             for (int c = 0; c < 4; ++c) {
-                const T wm = arm_at(arm, cs, c, e0 + stride), w0 = arm_at(arm, cs, c, e0 + 2 * stride);
-                const T w1 = arm_at(arm, cs, c, e0 + 3 * stride), wp = arm_at(arm, cs, c, e0 + 4 * stride);
+                T wm, w0, w1, wp;
+                if constexpr (kNear) {
+                    wm = arm[c * cs + off[1]]; w0 = arm[c * cs + off[2]]; w1 = arm[c * cs + off[3]]; wp = arm[c * cs + off[4]];
+                } else {
+                    wm = arm_at(arm, cs, c, e0 + stride); w0 = arm_at(arm, cs, c, e0 + 2 * stride);
+                    w1 = arm_at(arm, cs, c, e0 + 3 * stride); wp = arm_at(arm, cs, c, e0 + 4 * stride);
+                }
                 if (cf.spatial == PDM1_SPATIAL_FIRST_ORDER) {   // first_order.py:66-111
                     L[c] = w0;
                     R[c] = w1;
@@ -384,12 +449,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
             }
         }
         if constexpr (kNear) {
-            face_flux64(L, R, axis, unit, s.F + f, NF);
+            face_flux64(L, R, axis, unit, s.F + slot, NF);
         } else {
             T F[4];
             face_flux_f32x2(L, R, axis, unit, F);
 #pragma unroll
-            for (int c = 0; c < 4; ++c) s.F[c * NF + f] = F[c];
+            for (int c = 0; c < 4; ++c) s.F[c * NF + slot] = F[c];
         }
     }
     __syncthreads();
@@ -434,7 +499,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
             double un[4];
             if ((MODE == MODE_A || MODE == MODE_EULER) && sizeof(T) == sizeof(double)) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) un[c] = double(s.X[((c * (TX + 6) + (i + 3)) * TY + j) * TZ + k]);
+                for (int c = 0; c < 4; ++c) un[c] = double(s.X[c * kCells + ((i + 3) * TY + j) * TZ + k]);
             } else if (MODE == MODE_A || MODE == MODE_EULER) {
                 load_cell<MODE>(cf, co, d, Ua, li, lj, lk, un);   // the state in double
             } else {
@@ -499,7 +564,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
                     div4(unew, co.S1[m]);
                     project64(unew);
                     if constexpr (sizeof(T) == sizeof(double)) {
-                        double u2c = double(s.X[((0 * (TX + 6) + (i + 3)) * TY + j) * TZ + k]);
+                        double u2c = double(s.X[((i + 3) * TY + j) * TZ + k]);
                         double q2 = u2c * co.S2[m];
                         ed = dE * (qb[o] + 2.0 / 3.0 * q2);
                     } else {
@@ -582,15 +647,22 @@ __global__ void __launch_bounds__(NT, sizeof(T) == sizeof(double) ? 2 : 4) stage
             __syncthreads();
         }
     }
-    // tiles of all marching beams, back to back (one beam: its domain's tiles)
+    // tiles of all marching beams, back to back (one beam: its domain's tiles).  A CTA takes
+    // the first by its index and each further one from the stage's counter while it works
+    // on the one before: ragged tiles and those at the entrance cost less and more than the rest.
     const int total = MODE == MODE_RHS ? a.st[0].dom.ntiles : cf.tile_off[cf.nbeams];
-    for (int gt = blockIdx.x; gt < total; gt += gridDim.x) {
+    int *const counter = cf.tile_off + cf.nbeams + 1 + (MODE == MODE_EULER ? 0 : MODE);
+    for (int gt = blockIdx.x; gt < total;) {
         const int b = (MODE == MODE_RHS || cf.nbeams == 1) ? 0 : beam_of_tile(cf.tile_off, cf.nbeams, gt);
         const int tile = MODE == MODE_RHS ? gt : gt - cf.tile_off[b];
+        int next = gridDim.x + gt;
+        if (MODE != MODE_RHS && threadIdx.x == 0 && total > (int)gridDim.x) next = gridDim.x + atomicAdd(counter, 1);
         const DomainDev d = a.st[b].dom;
         stage_tile<T, MODE, Tl, LEARN>(a, cf, d, b, tile, bar_phase, cta_inv);
-        bar_phase ^= 1u;
+        if (threadIdx.x == 0) sh.next_tile[bar_phase] = next;
         __syncthreads();   // shared memory is reused by the next tile
+        gt = sh.next_tile[bar_phase];
+        bar_phase ^= 1u;
     }
     if (MODE == MODE_C && !cf.moving) block_max_atomic<NT>(cta_inv, &a.st[0].inv_bits);
 }
