@@ -242,10 +242,9 @@ constexpr int NT = 256;   // threads of a stage CTA
 
 // A tile shape: the tile's cells, its cross-shaped 3-cell WENO halo (no
 // corners: WENO reads along one axis at a time) and its faces.  Shared memory
-// holds, in float, three arms per component, each the core plus the halo along
-// one axis (the core stored three times), so every 6-point stencil is a strided
-// run in one arm; in double one copy of every cell (the x arm, then the y and z
-// halos): a third less, so that three CTAs fit an SM.
+// holds three arms per component, each the core plus the halo along one axis
+// (the core stored three times), so every 6-point stencil is a strided run in
+// one arm.
 template <int X, int Y, int Z>
 struct Tile {
     static constexpr int CELLS = X * Y * Z;
@@ -261,7 +260,7 @@ struct Tile {
     static constexpr int AZ = X * Y * (Z + 6);
     template <typename T>
     static constexpr size_t arm_bytes() {
-        return sizeof(T) * 4 * ((sizeof(T) == sizeof(double) ? SX + SY + SZ : AX + AY + AZ) + NF);
+        return sizeof(T) * 4 * (AX + AY + AZ + NF);
     }
 };
 

@@ -168,10 +168,6 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
     s.Y = s.X + 4 * AX;    // [c][i][j + 3][k]
     s.Z = s.Y + 4 * AY;    // [c][i][j][k + 3]
     s.F = s.Z + 4 * AZ;
-    // double: component c at s.X + c * kCells: [i + 3][j][k], the y halo [i][0..2 | 3..5][k]
-    // from kHaloY on, the z halo [i][j][0..2 | 3..5] from kHaloZ on
-    constexpr int kCells = SX + SY + SZ, kHaloY = SX, kHaloZ = SX + SY;
-    if constexpr (kNear) s.F = s.X + 4 * kCells;
     int tid = threadIdx.x;
     asm volatile("" : "+r"(tid));   // the indices that follow from it are formed per tile: hoisted, they spill
     const bool unit = cf.unit_speeds != 0;
@@ -240,19 +236,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         load_cell<MODE>(cf, co, d, src, i0 + ii - 3, j0 + j, k0 + k, u);
         const bool core = ii >= 3 && ii < TX + 3;
         const int ex = (ii * TY + j) * TZ + k;
-        if constexpr (kNear) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                out_of_range |= !weno_range(u[c]);
-                s.X[c * kCells + ex] = u[c];
-            }
-            continue;
-        }
         const int ey = ((ii - 3) * (TY + 6) + j + 3) * TZ + k;
         const int ez = ((ii - 3) * TY + j) * (TZ + 6) + k + 3;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const T v = T(u[c]);
+            if constexpr (kNear) out_of_range |= !weno_range(u[c]);
             arm_at(s.X, AX, c, ex) = v;
             if (core) {
                 arm_at(s.Y, AY, c, ey) = v;
@@ -268,12 +257,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         load_cell<MODE>(cf, co, d, src, i0 + i, gj, k0 + k, u);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            if constexpr (kNear) {
-                out_of_range |= !weno_range(u[c]);
-                s.X[c * kCells + kHaloY + e] = u[c];
-            } else {
-                arm_at(s.Y, AY, c, (i * (TY + 6) + aj) * TZ + k) = T(u[c]);
-            }
+            if constexpr (kNear) out_of_range |= !weno_range(u[c]);
+            arm_at(s.Y, AY, c, (i * (TY + 6) + aj) * TZ + k) = T(u[c]);
         }
     }
     for (int e = tid; e < SZ; e += NT) {
@@ -285,12 +270,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         load_cell<MODE>(cf, co, d, src, i0 + i, j0 + j, gk, u);
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            if constexpr (kNear) {
-                out_of_range |= !weno_range(u[c]);
-                s.X[c * kCells + kHaloZ + e] = u[c];
-            } else {
-                arm_at(s.Z, AZ, c, (i * TY + j) * (TZ + 6) + ak) = T(u[c]);
-            }
+            if constexpr (kNear) out_of_range |= !weno_range(u[c]);
+            arm_at(s.Z, AZ, c, (i * TY + j) * (TZ + 6) + ak) = T(u[c]);
         }
     }
     }   // the double-precision source
@@ -305,11 +286,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
             if (li >= nx || lj >= ny) continue;
             T ui = T(boundary_value<MODE>(a, cf, bm, co, d, c, li, lj));
             const int ez = (i * TY + j) * (TZ + 6);
-            auto z = [&](int kk) -> T & {   // cell k0 - 3 + kk
-                if constexpr (kNear)
-                    return s.X[c * kCells + (kk < 3 ? kHaloZ + (i * TY + j) * 6 + kk : ((i + 3) * TY + j) * TZ + kk - 3)];
-                else return arm_at(s.Z, AZ, c, ez + kk);
-            };
+            auto z = [&](int kk) -> T & { return arm_at(s.Z, AZ, c, ez + kk); };
             T u0 = z(3), u1 = z(4), u2 = z(5), u3 = z(6);
             if (cf.spatial == PDM1_SPATIAL_WENO_Z) {   // quartic, boundary.py:247-320
                 z(2) = T(5.0) * ui - T(77.0 / 12.0) * u0 + T(43.0 / 12.0) * u1 - T(17.0 / 12.0) * u2 + T(0.25) * u3;
@@ -360,19 +337,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         // the six cells along the axis, i - 3 .. i + 2 (face between i - 1 and i),
         // are arm indices i .. i + 5
         T *arm = s.X;
-        int e0 = 0, stride = 0, cs = kCells, off[6];
-        if constexpr (kNear) {
-            const int pos = axis == 0 ? i : (axis == 1 ? j : k), n = axis == 1 ? TY : TZ;
-            const int st = axis == 0 ? TY * TZ : (axis == 1 ? TZ : 1);
-            const int c0 = axis == 0 ? j * TZ + k : (axis == 1 ? (i + 3) * TY * TZ + k : ((i + 3) * TY + j) * TZ);
-            const int h0 = axis == 1 ? kHaloY + i * 6 * TZ + k : kHaloZ + (i * TY + j) * 6;
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                const int p = pos - 3 + q;
-                const bool core = axis == 0 || (p >= 0 && p < n);
-                off[q] = core ? c0 + (axis == 0 ? p + 3 : p) * st : h0 + (p < 0 ? p + 3 : p - n + 3) * st;
-            }
-        } else if (axis == 0) {
+        int e0, stride, cs;
+        if (axis == 0) {
             arm = s.X; e0 = (i * TY + j) * TZ + k; stride = TY * TZ; cs = AX;
         } else if (axis == 1) {
             arm = s.Y; e0 = (i * (TY + 6) + j) * TZ + k; stride = TZ; cs = AY;
@@ -404,14 +370,14 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
                     for (int c = 0; c < 4; ++c) {
                         T w[6];
 #pragma unroll
-                        for (int q = 0; q < 6; ++q) w[q] = arm[c * cs + off[q]];
+                        for (int q = 0; q < 6; ++q) w[q] = arm[e0 + c * cs + q * stride];
                         weno_pair(w, L[c], R[c]);
                     }
                 } else {
                     for (int c = 0; c < 4; ++c) {
                         T w[6];
 #pragma unroll
-                        for (int q = 0; q < 6; ++q) w[q] = arm[c * cs + off[q]];
+                        for (int q = 0; q < 6; ++q) w[q] = arm[e0 + c * cs + q * stride];
                         const T l = weno_left_ieee(w[0], w[1], w[2], w[3], w[4]);
                         const T r = weno_left_ieee(w[5], w[4], w[3], w[2], w[1]);
 #pragma unroll
@@ -423,13 +389,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         } else {
             // the narrower stencils read cells i-2 .. i+1 (arm indices i+1 .. i+4)
             for (int c = 0; c < 4; ++c) {
-                T wm, w0, w1, wp;
-                if constexpr (kNear) {
-                    wm = arm[c * cs + off[1]]; w0 = arm[c * cs + off[2]]; w1 = arm[c * cs + off[3]]; wp = arm[c * cs + off[4]];
-                } else {
-                    wm = arm_at(arm, cs, c, e0 + stride); w0 = arm_at(arm, cs, c, e0 + 2 * stride);
-                    w1 = arm_at(arm, cs, c, e0 + 3 * stride); wp = arm_at(arm, cs, c, e0 + 4 * stride);
-                }
+                const T wm = arm_at(arm, cs, c, e0 + stride), w0 = arm_at(arm, cs, c, e0 + 2 * stride);
+                const T w1 = arm_at(arm, cs, c, e0 + 3 * stride), wp = arm_at(arm, cs, c, e0 + 4 * stride);
                 if (cf.spatial == PDM1_SPATIAL_FIRST_ORDER) {   // first_order.py:66-111
                     L[c] = w0;
                     R[c] = w1;
@@ -499,7 +460,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
             double un[4];
             if ((MODE == MODE_A || MODE == MODE_EULER) && sizeof(T) == sizeof(double)) {
 #pragma unroll
-                for (int c = 0; c < 4; ++c) un[c] = double(s.X[c * kCells + ((i + 3) * TY + j) * TZ + k]);
+                for (int c = 0; c < 4; ++c) un[c] = double(s.X[((c * (TX + 6) + (i + 3)) * TY + j) * TZ + k]);
             } else if (MODE == MODE_A || MODE == MODE_EULER) {
                 load_cell<MODE>(cf, co, d, Ua, li, lj, lk, un);   // the state in double
             } else {
