@@ -109,7 +109,8 @@ typedef struct {
     int graph_replays;        /* CUDA graph launches used by the march */
     int kernel_launches;      /* kernels this library launched for the march */
     int stage_launches;       /* launches of the fused stage kernels */
-    double stage_ms;          /* their summed device time (CUDA events on the march stream) */
+    double stage_ms;          /* their summed device time, per step from the first stage's
+                              * start to the last one's end (the device's nanosecond clock) */
     double cell_steps;        /* sum over energy steps of the cells marched */
     double max_box_cells;     /* largest domain (cells) one beam marched in one step */
     int box_grow_events;      /* learned box: faces grown by the outgoing-flux check */

@@ -70,10 +70,15 @@ struct BeamDev {
     DomainDev init_box;             // moving_active_domain.py:35-60
 };
 
+constexpr int kStepsPerGraph = 32;
+
 // What the host polls between graph replays.
 struct MarchSummary {
     int active;         // beams that marched in the last step
     int error;          // OR of the beams' error flags
+    // per step of the replay: the nanosecond clock when the first stage's first CTA begins
+    // and when the last stage's last CTA ends
+    unsigned long long begin_ns[kStepsPerGraph], end_ns[kStepsPerGraph];
 };
 
 struct ConfigDev {
@@ -312,6 +317,7 @@ struct StageArgs {
     double *dose;       // accumulated dose (full grid), or NULL
     double *edep;       // when non-NULL: energy deposition written instead of dose
     double *snap;       // snapshot buffer base (slot * 4N, full grid)
+    unsigned long long *begin_ns, *end_ns;   // stage timing of this step, or NULL
     double *rhs_out;    // MODE_RHS output
     const double *bc_plane;   // MODE_RHS: explicit z-min boundary state (4,nx,ny)
     double rhs_energy_density;

@@ -592,6 +592,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
     }
 }
 
+__device__ __forceinline__ unsigned long long clock_ns() {
+    unsigned long long v;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(v));
+    return v;
+}
+
 // LEARN (stage C of a plan with a learned box): the tile's fluence moments of
 // the new state are accumulated for the next step's proposer.
 template <typename T, int MODE, class Tl, bool LEARN = false>
@@ -600,6 +606,8 @@ __global__ void __launch_bounds__(NT, sizeof(T) == sizeof(double) ? 2 : 4) stage
     extern __shared__ __align__(16) unsigned char smem_raw[];
     StageShared &sh = *reinterpret_cast<StageShared *>(smem_raw);
     double cta_inv = 0.0;
+    if ((MODE == MODE_A || MODE == MODE_EULER) && a.begin_ns && blockIdx.x == 0 && threadIdx.x == 0)
+        *a.begin_ns = *a.end_ns = clock_ns();
     // FP32 stages B and C: bulk copies of the float4 stage state, one mbarrier phase per tile
     unsigned bar_phase = 0;
     if constexpr (kF4Source<T, MODE>) {
@@ -626,6 +634,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == sizeof(double) ? 2 : 4) stage
         bar_phase ^= 1u;
     }
     if (MODE == MODE_C && !cf.moving) block_max_atomic<NT>(cta_inv, &a.st[0].inv_bits);
+    if ((MODE == MODE_C || MODE == MODE_EULER) && a.end_ns && threadIdx.x == 0) atomicMax(a.end_ns, clock_ns());
 }
 
 }  // namespace pdm1
