@@ -166,10 +166,11 @@ __device__ __forceinline__ double gauss_point(double E, double dE, int p) {
 }
 
 // One CTA per beam, latency-bound: one thread decides the step, one thread takes each
-// table look-up (its loads issued together, table_dev), one thread each exponential with
-// the optical depth it needs.  Before, a thread took three look-ups in turn, one thread a
-// material's four depths, and each look-up a double logarithm (17.1 -> 14.0 us with cold
-// caches, 12x12x100 march 22.6 -> 20.9 ms).
+// table look-up (its loads issued together, table_dev; the tables' views and what the
+// decision reads are loaded ahead), one thread each exponential with the optical depth it
+// needs.  All lanes of a warp take one path through a look-up: split by coefficient they ran
+// one after the other, 7400 of the kernel's 14600 cycles.  Before, a thread took three
+// look-ups in turn, one thread a material's four depths, and each look-up a double logarithm.
 __global__ void __launch_bounds__(256) prologue_kernel(const ConfigDev *cfp, Coeffs *cos,
                                                        MarchState *sts, double *energies) {
     const ConfigDev &cf = *cfp;
@@ -182,36 +183,52 @@ __global__ void __launch_bounds__(256) prologue_kernel(const ConfigDev *cfp, Coe
     __shared__ int sActive;
     __shared__ double eS[kMaxMat][kEvalS], eTr[kMaxMat][8], eNu[kMaxMat][8];
     const int t = threadIdx.x;
+    // the first look-up's table, and what the decision reads, are on their way together
+    const int nm = cf.nm, per = nm * kEvalPerMat;
+    auto table_of = [&](int w) -> const TableView & {
+        const MatDev &m = cf.mats[w / kEvalPerMat];
+        const int q = w % kEvalPerMat;
+        return q < kEvalS ? m.sp : (q < kEvalS + 8 ? m.tr : m.nuc);
+    };
+    TableView view = table_of(t < per ? t : 0);
+    const bool linear = cf.interp == PDM1_INTERP_LINEAR, nuclear = cf.nuclear != 0;
+    const int scattering = cf.scattering;
     if (t == 0) {
         int active = 0, slot = -1;
         const double E = st->E, forced = st->forced_dE;
         const double inv = __longlong_as_double((long long)st->inv_bits);
         const int done = st->done, step0 = st->step, ti = st->ti, taken = st->taken;
         const double cells = (double)st->dom.nx * st->dom.ny * st->dom.nz;
-        const int ntiles = st->dom.ntiles;
+        const double cells0 = st->cell_steps, most = st->max_cells;
+        const int ntiles = st->dom.ntiles, nbeams = cf.nbeams, n_targets = cf.n_targets, n_schedule = cf.n_schedule;
+        const int step_limit = cf.step_limit, max_steps = cf.max_steps;
+        const double Emin = cf.Emin, cfl = cf.cfl, max_dE = cf.max_dE;
+        const double *const schedule = cf.schedule, *const targets = cf.targets;
+        int *const tile_off = cf.tile_off;
+        MarchSummary *const summary = cf.summary;
         int error = st->error;
         double dE = 0.0, En = E;
         if (!done && error == 0) {
-            if (!(E > cf.Emin) || (cf.step_limit >= 0 && step0 >= cf.step_limit)) {
+            if (!(E > Emin) || (step_limit >= 0 && step0 >= step_limit)) {
                 st->done = 1;
-            } else if (step0 >= cf.max_steps) {
+            } else if (step0 >= max_steps) {
                 error |= ERR_DEV_MAXSTEPS;
                 st->done = 1;
             } else {
                 if (forced > 0.0) {
                     dE = forced;
-                } else if (cf.schedule) {
+                } else if (schedule) {
                     // a prescribed energy schedule (another run's steps): the
                     // next energy is taken as given, past its end down to Emin
-                    dE = step0 + 1 < cf.n_schedule ? E - cf.schedule[step0 + 1] : E - cf.Emin;
+                    dE = step0 + 1 < n_schedule ? E - schedule[step0 + 1] : E - Emin;
                 } else {
-                    dE = cf.cfl / inv;
-                    dE = cf.max_dE < dE ? cf.max_dE : dE;
-                    if (ti < cf.n_targets) {
-                        double tg = cf.targets[ti];
+                    dE = cfl / inv;
+                    dE = max_dE < dE ? max_dE : dE;
+                    if (ti < n_targets) {
+                        double tg = targets[ti];
                         if (E > tg && tg >= E - dE) dE = E - tg;
                     }
-                    if (E - cf.Emin < dE) dE = E - cf.Emin;
+                    if (E - Emin < dE) dE = E - Emin;
                 }
                 if (!(dE > 0.0) || !isfinite(dE)) {
                     error |= ERR_DEV_NONFINITE;
@@ -219,18 +236,18 @@ __global__ void __launch_bounds__(256) prologue_kernel(const ConfigDev *cfp, Coe
                 } else {
                     active = 1;
                     En = E - dE;
-                    if (cf.schedule && forced <= 0.0 && step0 + 1 < cf.n_schedule) En = cf.schedule[step0 + 1];
+                    if (schedule && forced <= 0.0 && step0 + 1 < n_schedule) En = schedule[step0 + 1];
                     const int step = step0 + 1;
                     if (energies) energies[step] = En;
-                    if (ti < cf.n_targets && fabs(En - cf.targets[ti]) <= 1e-12) {
+                    if (ti < n_targets && fabs(En - targets[ti]) <= 1e-12) {
                         slot = taken;
                         st->taken = taken + 1;
                         st->ti = ti + 1;
                     }
                     st->step = step;
                     st->E = En;
-                    st->cell_steps += cells;
-                    st->max_cells = fmax(st->max_cells, cells);
+                    st->cell_steps = cells0 + cells;
+                    st->max_cells = fmax(most, cells);
                     st->inv_bits = 0ull;
                     if (forced > 0.0) st->done = 1;
                 }
@@ -239,40 +256,37 @@ __global__ void __launch_bounds__(256) prologue_kernel(const ConfigDev *cfp, Coe
         }
         sE = E; sdE = dE; sActive = active;
         co->E = E; co->dE = dE; co->E_next = En; co->active = active; co->snap_slot = slot;
-        if (cf.nbeams == 1) {
-            cf.tile_off[0] = 0;
-            cf.tile_off[1] = active ? ntiles : 0;
-            for (int q = 0; q < kTileCounters; ++q) cf.tile_off[2 + q] = 0;
-            cf.summary->active = active;
-            cf.summary->error = error;
+        if (nbeams == 1) {
+            tile_off[0] = 0;
+            tile_off[1] = active ? ntiles : 0;
+            for (int q = 0; q < kTileCounters; ++q) tile_off[2 + q] = 0;
+            summary->active = active;
+            summary->error = error;
         }
     }
     __syncthreads();
     if (!sActive) return;
     const double E = sE, dE = sdE;
-    const int nm = cf.nm;
-    for (int w = t; w < nm * kEvalPerMat; w += 256) {
+    // every lane of a warp takes the same path: its own table at its own energy
+    for (int w = t; w < per; w += 256) {
         const int m = w / kEvalPerMat, q = w % kEvalPerMat;
-        const MatDev &mat = cf.mats[m];
-        bool ok = true;
-        if (q < kEvalS) {
-            const double e = q == 0 ? E : (q == 1 ? E - dE / 3.0 : (q == 2 ? E - 2.0 * dE / 3.0 : (q == 3 ? E - dE :
-                             (q == 4 ? E - 0.5 * dE : gauss_point(E, dE, q - 5)))));
-            double s = 1.0;
-            ok = stopping_power_dev(mat, e, s);
-            eS[m][q] = s;
+        if (w != t) view = table_of(w);
+        double e;
+        if (q < 5) {
+            const double part = q == 1 ? dE / 3.0 : (q == 2 ? 2.0 * dE / 3.0 : (q == 3 ? dE : 0.5 * dE));
+            e = q == 0 ? E : E - part;
         } else {
-            const int p = (q - kEvalS) & 7;
-            const double e = gauss_point(E, dE, p);
-            double v = 0.0;
-            if (q < kEvalS + 8) {
-                ok = transport_dev(cf, mat, e, v);
-                eTr[m][p] = v;
-            } else {
-                if (cf.nuclear) ok = nuclear_dev(cf, mat, e, v);
-                eNu[m][p] = v;
-            }
+            e = gauss_point(E, dE, q < kEvalS ? q - 5 : (q - kEvalS) & 7);
         }
+        const bool is_S = q < kEvalS, is_tr = !is_S && q < kEvalS + 8;
+        double v = is_S ? 1.0 : 0.0;
+        bool ok = true;
+        if (is_S || (is_tr ? scattering == PDM1_SCATTERING_WENTZEL : nuclear))
+            ok = table_dev(view, is_S || !linear, e, v);
+        else if (is_tr) ok = transport_dev(cf, cf.mats[m], e, v);   // Rossi's formula, or none
+        if (is_S) eS[m][q] = v;
+        else if (is_tr) eTr[m][q - kEvalS] = v;
+        else eNu[m][q - kEvalS - 8] = v;
         if (!ok) atomicOr(&st->error, ERR_DEV_RANGE);
     }
     __syncthreads();
