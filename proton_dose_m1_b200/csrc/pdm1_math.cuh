@@ -178,7 +178,12 @@ __device__ __forceinline__ float2 pk_fma(float2 a, float2 b, float2 c) { return 
 __device__ __forceinline__ float2 pk_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 pk_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
 // approximate reciprocal per lane (MUFU), within 2 ulp for |x| below 2^126
-__device__ __forceinline__ float2 pk_rcp(float2 x) { return make_float2(__fdividef(1.0f, x.x), __fdividef(1.0f, x.y)); }
+__device__ __forceinline__ float rcp_f32(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float2 pk_rcp(float2 x) { return make_float2(rcp_f32(x.x), rcp_f32(x.y)); }
 __device__ __forceinline__ float2 pk_sqrt(float2 x) { return make_float2(sqrtf(x.x), sqrtf(x.y)); }
 
 // Jiang-Shu smoothness indicator 13/12 a^2 + 1/4 b^2
@@ -195,24 +200,21 @@ __device__ __forceinline__ float2 weno_left_f32x2(float2 v0, float2 v1, float2 v
     const float2 beta1 = pk_beta(pk_add(pk_fma(pk(-2.0f), v2, v1), v3), pk_fma(pk(-1.0f), v3, v1));
     const float2 beta2 = pk_beta(pk_add(pk_fma(pk(-2.0f), v3, v2), v4),
                                  pk_fma(pk(-4.0f), v3, pk_fma(pk(3.0f), v2, v4)));
+    // tau5 = |d|; the sign goes with the absolute value of the ratios, free in the minimum
     const float2 d = pk_fma(pk(-1.0f), beta0, beta2);
-    const float2 tau5 = make_float2(fabsf(d.x), fabsf(d.y));
     const float2 eps = pk(float(kWenoEps));
-    float2 r0 = pk_mul(tau5, pk_rcp(pk_add(beta0, eps)));
-    float2 r1 = pk_mul(tau5, pk_rcp(pk_add(beta1, eps)));
-    float2 r2 = pk_mul(tau5, pk_rcp(pk_add(beta2, eps)));
-    r0 = make_float2(fminf(r0.x, 1e30f), fminf(r0.y, 1e30f));
-    r1 = make_float2(fminf(r1.x, 1e30f), fminf(r1.y, 1e30f));
-    r2 = make_float2(fminf(r2.x, 1e30f), fminf(r2.y, 1e30f));
+    auto held = [](float2 r) { return make_float2(fminf(fabsf(r.x), 1e30f), fminf(fabsf(r.y), 1e30f)); };
+    float2 t0 = held(pk_mul(d, pk_rcp(pk_add(beta0, eps))));
+    float2 t1 = held(pk_mul(d, pk_rcp(pk_add(beta1, eps))));
+    float2 t2 = held(pk_mul(d, pk_rcp(pk_add(beta2, eps))));
     // alpha_k / s^2 = d_k (s^-2 + (r_k / s)^2) with s = max r where r^2 could overflow, else s = 1
-    float2 sc = pk(1.0f);
-    const float mx = fmaxf(r0.x, fmaxf(r1.x, r2.x)), my = fmaxf(r0.y, fmaxf(r1.y, r2.y));
+    float2 e = pk(1.0f);
+    const float mx = fmaxf(t0.x, fmaxf(t1.x, t2.x)), my = fmaxf(t0.y, fmaxf(t1.y, t2.y));
     if (mx > 1e15f || my > 1e15f) {
-        if (mx > 1e15f) sc.x = __fdividef(1.0f, mx);
-        if (my > 1e15f) sc.y = __fdividef(1.0f, my);
+        const float2 sc = make_float2(mx > 1e15f ? rcp_f32(mx) : 1.0f, my > 1e15f ? rcp_f32(my) : 1.0f);
+        e = pk_mul(sc, sc);
+        t0 = pk_mul(t0, sc); t1 = pk_mul(t1, sc); t2 = pk_mul(t2, sc);
     }
-    const float2 e = pk_mul(sc, sc);
-    const float2 t0 = pk_mul(r0, sc), t1 = pk_mul(r1, sc), t2 = pk_mul(r2, sc);
     const float2 al0 = pk_mul(pk(0.1f), pk_fma(t0, t0, e));
     const float2 al1 = pk_mul(pk(0.6f), pk_fma(t1, t1, e));
     const float2 al2 = pk_mul(pk(0.3f), pk_fma(t2, t2, e));
@@ -563,8 +565,7 @@ __device__ __forceinline__ void face_flux_f32x2(const float L[4], const float R[
     const float2 r = pk_sqrt(pk_fma(pk(3.0f), q, one));
     float2 iso = pk_mul(q, pk_rcp(pk_add(r, one)));
     float2 dir = pk_fma(pk(-1.0f), r, pk(2.0f));
-    const float2 rjn = make_float2(jn.x > 0.0f ? __fdividef(1.0f, jn.x) : 0.0f,
-                                   jn.y > 0.0f ? __fdividef(1.0f, jn.y) : 0.0f);
+    const float2 rjn = make_float2(jn.x > 0.0f ? rcp_f32(jn.x) : 0.0f, jn.y > 0.0f ? rcp_f32(jn.y) : 0.0f);
     const float2 nx = pk_mul(jx, rjn), ny = pk_mul(jy, rjn), nz = pk_mul(jz, rjn);
     const float2 na = axis == 0 ? nx : (axis == 1 ? ny : nz);
     const float2 ja = axis == 0 ? jx : (axis == 1 ? jy : jz);
@@ -573,9 +574,9 @@ __device__ __forceinline__ void face_flux_f32x2(const float L[4], const float R[
     const float2 pi = pk_mul(phi, iso);   // the isotropic pressure on the normal component
     float2 Fc[4];
     Fc[0] = ja;
-    Fc[1] = axis == 0 ? pk_fma(pdn, nx, pi) : pk_mul(pdn, nx);
-    Fc[2] = axis == 1 ? pk_fma(pdn, ny, pi) : pk_mul(pdn, ny);
-    Fc[3] = axis == 2 ? pk_fma(pdn, nz, pi) : pk_mul(pdn, nz);
+    Fc[1] = pk_fma(pdn, nx, axis == 0 ? pi : pk(0.0f));
+    Fc[2] = pk_fma(pdn, ny, axis == 1 ? pi : pk(0.0f));
+    Fc[3] = pk_fma(pdn, nz, axis == 2 ? pi : pk(0.0f));
     float sl = -1.0f, sr = 1.0f;
     if (!unit_speeds) {
         // exact wave speeds; below the eigenvalue floor of phi the closure is
