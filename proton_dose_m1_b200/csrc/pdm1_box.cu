@@ -324,7 +324,7 @@ __device__ void mlp_warp16(const BoxModelDev &M, const __nv_bfloat16 *x, __nv_bf
 __global__ void __launch_bounds__(NT) box_moments_kernel(const ConfigDev *cfp, const MarchState *sts, int record) {
     const ConfigDev &cf = *cfp;
     __shared__ double part[NT / 32][ACC_MAX + 1];
-    __shared__ double pl[kMaxTileZ];
+    __shared__ double pl[NT / 32][kMaxTileZ];
     __shared__ double buf[NT];
     const int tid = threadIdx.x;
     const int total = record ? sts[0].dom.ntiles : cf.tile_off[cf.nbeams];
@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(NT) box_moments_kernel(const ConfigDev *cfp, c
             __syncthreads();
             tile_slab_max(cf, cf.slab, d, buf, i0, j0, k0);
         }
-        tile_moments_cta(cf, b, d, k0, valid, li, lj, lk, u, part, pl);
+        tile_moments_cta(cf, b, d, i0, j0, k0, valid, li, lj, lk, u, part, pl);
     }
 }
 

@@ -453,7 +453,7 @@ __device__ __forceinline__ void atomic_max_double(unsigned long long *target, do
     if (v > 0.0) atomicMax(target, (unsigned long long)__double_as_longlong(v));
 }
 
-// Per-slab maxima of phi over one tile (moving box): cell values in `buf`
+// The recorder's per-slab maxima of phi over one tile: cell values in `buf`
 // (one per cell of the tile, (i, j, k) with k fastest; -1 outside the box).
 __device__ __forceinline__ void tile_slab_max(const ConfigDev &cf, unsigned long long *slab, const DomainDev &d,
                                               const double *buf, int i0, int j0, int k0) {
@@ -479,6 +479,52 @@ __device__ __forceinline__ void tile_slab_max(const ConfigDev &cf, unsigned long
     }
 }
 
+// Per-slab maxima of phi over one stage tile (moving box) from each thread's value
+// (-1 outside the box): warp maxima over k, over j and k, and over j, then the few
+// values per slab from shared memory.  (One thread per slab reading the tile's 64
+// values in turn held the CTA for about 2000 cycles a tile.)
+template <class Tl>
+struct SlabScratch {
+    static constexpr int JL = Tl::TY < 32 / Tl::TZ ? Tl::TY : 32 / Tl::TZ;   // j values of a warp
+    double x[Tl::CELLS / (Tl::TZ * JL)], y[Tl::TX * Tl::TY], z[Tl::CELLS / 32][Tl::TZ];
+};
+template <class Tl>
+__device__ __forceinline__ void stage_slab_max(const ConfigDev &cf, unsigned long long *slab, const DomainDev &d,
+                                               double phi, int i0, int j0, int k0, SlabScratch<Tl> &s) {
+    constexpr int TX = Tl::TX, TY = Tl::TY, TZ = Tl::TZ, JL = SlabScratch<Tl>::JL;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    if (Tl::CELLS == NT || warp < Tl::CELLS / 32) {
+        double row = phi, z = phi;
+#pragma unroll
+        for (int w = 1; w < TZ; w <<= 1) row = fmax(row, __shfl_xor_sync(0xffffffffu, row, w));
+        double x = row;
+#pragma unroll
+        for (int w = TZ; w < TZ * JL; w <<= 1) x = fmax(x, __shfl_xor_sync(0xffffffffu, x, w));
+#pragma unroll
+        for (int w = TZ; w < 32; w <<= 1) z = fmax(z, __shfl_xor_sync(0xffffffffu, z, w));
+        if (lane % TZ == 0) s.y[t / TZ] = row;
+        if (lane % (TZ * JL) == 0) s.x[t / (TZ * JL)] = x;
+        if (lane < TZ) s.z[warp][lane] = z;
+    }
+    __syncthreads();
+    double m = 0.0;
+    if (t < TX) {
+#pragma unroll
+        for (int e = 0; e < TY / JL; ++e) m = fmax(m, s.x[t * (TY / JL) + e]);
+        if (i0 + t < d.nx) atomic_max_double(&slab[i0 + t], m);
+    } else if (t >= 32 && t < 32 + TY) {
+        const int j = t - 32;
+#pragma unroll
+        for (int i = 0; i < TX; ++i) m = fmax(m, s.y[i * TY + j]);
+        if (j0 + j < d.ny) atomic_max_double(&slab[cf.nx + j0 + j], m);
+    } else if (t >= 64 && t < 64 + TZ) {
+        const int k = t - 64;
+#pragma unroll
+        for (int w = 0; w < Tl::CELLS / 32; ++w) m = fmax(m, s.z[w][k]);
+        if (k0 + k < d.nz) atomic_max_double(&slab[cf.nx + cf.ny + k0 + k], m);
+    }
+}
+
 // Beam owning global tile t of the step: tile_off holds the exclusive prefix
 // sums of the beams' tile counts (beams that do not march have none).
 __device__ __forceinline__ int beam_of_tile(const int *tile_off, int nbeams, int t) {
@@ -496,57 +542,75 @@ __device__ __forceinline__ unsigned long long *beam_slab(const ConfigDev &cf, in
 
 // Learned box: one tile's contribution to the beam's fluence moments, face
 // currents and z-plane currents (acc, plane) from the state u of each cell
-// (cell (li, lj, lk) of domain d, `valid` inside it).  Called by every thread
-// of a CTA of THREADS threads laid out as the stage tile (k fastest); `part` and
-// `pl` are shared scratch of THREADS/32 x (ACC_MAX + 1) and kMaxTileZ doubles.
+// (cell (li, lj, lk) of domain d, `valid` inside it; the tile begins at (i0, j0, k0)).
+// Called by every thread of a CTA of THREADS threads laid out as the stage tile (k
+// fastest, a power of two); `part` and `pl` are shared scratch.  The twelve sums go
+// through one butterfly that halves the values a lane holds as it doubles the lanes
+// they cover (16 exchanges of a double instead of 5 per sum); the face currents are
+// summed only in tiles that touch a face; a plane's current by the lanes that share k.
+// With 19 separate warp sums and one shared-memory atomic per cell the learned
+// stage C took 1.36 times the time of stage B on the 256x256x320 field.
 template <int THREADS = NT>
-__device__ __forceinline__ void tile_moments_cta(const ConfigDev &cf, int b, const DomainDev &d, int k0,
-                                                 bool valid, int li, int lj, int lk, const double u[4],
-                                                 double (*part)[ACC_MAX + 1], double *pl) {
-    constexpr int kSums = ACC_MAX;   // summed entries; max phi separately
+__device__ __forceinline__ void tile_moments_cta(const ConfigDev &cf, int b, const DomainDev &d, int i0, int j0,
+                                                 int k0, bool valid, int li, int lj, int lk, const double u[4],
+                                                 double (*part)[ACC_MAX + 1], double (*pl)[kMaxTileZ]) {
+    constexpr int kSums = ACC_MAX, kPlain = ACC_FACE, WARPS = THREADS / 32;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int kk = tid % d.tz;
-    if (tid < d.tz) pl[tid] = 0.0;
-    double v[kSums + 1];
-#pragma unroll
-    for (int q = 0; q <= kSums; ++q) v[q] = 0.0;
-    if (valid) {
-        const double phi = u[0], jx = u[1], jy = u[2], jz = u[3];
+    const bool faces = (i0 == 0 && d.i0 > 0) || (i0 + d.tx >= d.nx && d.i0 + d.nx < cf.nx) ||
+                       (j0 == 0 && d.j0 > 0) || (j0 + d.ty >= d.ny && d.j0 + d.ny < cf.ny) ||
+                       (k0 == 0 && d.k0 > 0) || (k0 + d.tz >= d.nz && d.k0 + d.nz < cf.nz);
+    const double phi = valid ? u[0] : 0.0, jx = valid ? u[1] : 0.0, jy = valid ? u[2] : 0.0, jz = valid ? u[3] : 0.0;
+    double m = phi;
+    {
         const double gx = d.i0 + li + 0.5, gy = d.j0 + lj + 0.5, gz = d.k0 + lk + 0.5;
-        v[ACC_M] = phi;
-        v[ACC_X] = phi * gx; v[ACC_X + 1] = phi * gy; v[ACC_X + 2] = phi * gz;
-        v[ACC_X2] = phi * gx * gx; v[ACC_X2 + 1] = phi * gy * gy; v[ACC_X2 + 2] = phi * gz * gz;
-        v[ACC_J] = jx; v[ACC_J + 1] = jy; v[ACC_J + 2] = jz;
-        v[ACC_JABS] = fabs(jx); v[ACC_JABS + 1] = fabs(jy);
-        if (li == 0 && d.i0 > 0) v[ACC_FACE + 0] = fabs(jx);
-        if (li == d.nx - 1 && d.i0 + d.nx < cf.nx) v[ACC_FACE + 1] = fabs(jx);
-        if (lj == 0 && d.j0 > 0) v[ACC_FACE + 2] = fabs(jy);
-        if (lj == d.ny - 1 && d.j0 + d.ny < cf.ny) v[ACC_FACE + 3] = fabs(jy);
-        if (lk == 0 && d.k0 > 0) v[ACC_FACE + 4] = fabs(jz);
-        if (lk == d.nz - 1 && d.k0 + d.nz < cf.nz) v[ACC_FACE + 5] = fabs(jz);
-        v[kSums] = phi;
-    }
-    __syncthreads();   // pl zeroed
-    atomicAdd(&pl[kk], v[ACC_J + 2]);
+        const double px = phi * gx, py = phi * gy, pz = phi * gz;
+        double v[16] = {phi, px, py, pz, px * gx, py * gy, pz * gz, jx, jy, jz, fabs(jx), fabs(jy), 0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-    for (int q = 0; q < kSums; ++q)
-        for (int w = 16; w > 0; w >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], w);
-    for (int w = 16; w > 0; w >>= 1) v[kSums] = fmax(v[kSums], __shfl_xor_sync(0xffffffffu, v[kSums], w));
-    if (lane == 0)
-        for (int q = 0; q <= kSums; ++q) part[warp][q] = v[q];
+        for (int w = 8; w > 0; w >>= 1) {
+            const bool up = (lane & w) != 0;
+#pragma unroll
+            for (int q = 0; q < w; ++q) {
+                const double keep = up ? v[q + w] : v[q], send = up ? v[q] : v[q + w];
+                v[q] = keep + __shfl_xor_sync(0xffffffffu, send, w);
+            }
+        }
+        v[0] += __shfl_xor_sync(0xffffffffu, v[0], 16);   // lane l: the warp's sum of value l & 15
+        if (lane < kPlain) part[warp][lane] = v[0];
+    }
+    for (int w = 16; w > 0; w >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, w));
+    if (lane == 0) part[warp][kSums] = m;
+    if (faces) {
+        double f[6];
+        f[0] = li == 0 && d.i0 > 0 ? fabs(jx) : 0.0;
+        f[1] = li == d.nx - 1 && d.i0 + d.nx < cf.nx ? fabs(jx) : 0.0;
+        f[2] = lj == 0 && d.j0 > 0 ? fabs(jy) : 0.0;
+        f[3] = lj == d.ny - 1 && d.j0 + d.ny < cf.ny ? fabs(jy) : 0.0;
+        f[4] = lk == 0 && d.k0 > 0 ? fabs(jz) : 0.0;
+        f[5] = lk == d.nz - 1 && d.k0 + d.nz < cf.nz ? fabs(jz) : 0.0;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            for (int w = 16; w > 0; w >>= 1) f[q] += __shfl_xor_sync(0xffffffffu, f[q], w);
+            if (lane == 0) part[warp][ACC_FACE + q] = f[q];
+        }
+    }
+    double z = jz;
+    for (int w = d.tz; w < 32; w <<= 1) z += __shfl_xor_sync(0xffffffffu, z, w);
+    if (lane < d.tz) pl[warp][lane] = z;
     __syncthreads();
     double *acc = cf.acc + (size_t)b * kAcc;
-    if (tid < kSums) {
+    if (tid < (faces ? kSums : kPlain)) {
         double s = 0.0;
-        for (int w = 0; w < THREADS / 32; ++w) s += part[w][tid];
+        for (int w = 0; w < WARPS; ++w) s += part[w][tid];
         if (s != 0.0) atomicAdd(&acc[tid], s);
     } else if (tid == kSums) {
-        double m = 0.0;
-        for (int w = 0; w < THREADS / 32; ++w) m = fmax(m, part[w][kSums]);
+        m = 0.0;
+        for (int w = 0; w < WARPS; ++w) m = fmax(m, part[w][kSums]);
         atomic_max_double(reinterpret_cast<unsigned long long *>(&acc[ACC_MAX]), m);
     } else if (tid >= 32 && tid < 32 + d.tz) {
         const int k = tid - 32;
-        if (k0 + k < d.nz && pl[k] != 0.0) atomicAdd(&cf.plane[(size_t)b * cf.nz + d.k0 + k0 + k], pl[k]);
+        double s = 0.0;
+        for (int w = 0; w < WARPS; ++w) s += pl[w][k];
+        if (k0 + k < d.nz && s != 0.0) atomicAdd(&cf.plane[(size_t)b * cf.nz + d.k0 + k0 + k], s);
     }
     __syncthreads();
 }

@@ -140,9 +140,9 @@ __device__ __forceinline__ void patch_zmax(const DomainDev &d, int k0, float4 *Z
 // Shared memory of a stage CTA ahead of the tile's arms and fluxes (all of it
 // dynamic).
 struct StageShared {
-    double slab_buf[NT];             // moving box: phi of the tile's cells
+    double slab[208];                // moving box: the tile's slab maxima (SlabScratch)
     double mom_part[NT / 32][ACC_MAX + 1];   // learned box: moments of the new state
-    double mom_pl[kMaxTileZ];
+    double mom_pl[NT / 32][kMaxTileZ];
     unsigned long long stage_bar;    // FP32 stages B and C: the tile's bulk copies
     int next_tile[2];                // the CTA's next tile, by the parity of the tile it is on
 };
@@ -582,13 +582,12 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
         }
     }
     if (MODE == MODE_C && cf.moving) {
-        sh.slab_buf[tid] = phi_new;
-        __syncthreads();
-        tile_slab_max(cf, beam_slab(cf, b), d, sh.slab_buf, i0, j0, k0);
+        static_assert(sizeof(SlabScratch<Tl>) <= sizeof(sh.slab), "slab scratch");
+        stage_slab_max<Tl>(cf, beam_slab(cf, b), d, phi_new, i0, j0, k0, *reinterpret_cast<SlabScratch<Tl> *>(sh.slab));
     }
     if constexpr (LEARN && MODE == MODE_C) {
         // learned box: the moments of the new state feed the next step's proposer
-        tile_moments_cta<NT>(cf, b, d, k0, valid, li, lj, lk, um, sh.mom_part, sh.mom_pl);
+        tile_moments_cta<NT>(cf, b, d, i0, j0, k0, valid, li, lj, lk, um, sh.mom_part, sh.mom_pl);
     }
 }
 
