@@ -242,12 +242,14 @@ int pdm1_plan_set_staging(pdm1_plan *plan, int bulk);
 /* ---- Tile shape of the stage kernels ---------------------------------------
  * No reference counterpart.  The fused stage kernels are built for
  * PDM1_NUM_TILES tile shapes of 256 cells (one per thread): 4x8x8 (the
- * default), 8x8x4 and 2x8x16 (x, y, z; z is the contiguous axis).  The
- * autotuner marches the first `steps` energy steps of the plan's problem with
- * every shape (in scratch buffers it allocates; the plan's results are not
- * touched), measures the stage-kernel time per cell-step with CUDA events,
- * keeps the fastest shape for the plan and reports it in *best_tile and the
- * measurements in ns_per_cell_step (host, PDM1_NUM_TILES, may be NULL). */
+ * default), 8x8x4 and 2x8x16 (x, y, z; z is the contiguous axis).  A plan whose
+ * grids of all beams fit one wave of CTAs in 4x4x4 tiles runs on those under
+ * every setting (the results are the same doubles).  The autotuner marches the
+ * first `steps` energy steps of the plan's problem with every shape (in scratch
+ * buffers it allocates; the plan's results are not touched), measures the
+ * stage-kernel time per cell-step with the device's clock, keeps the fastest
+ * shape for the plan and reports it in *best_tile and the measurements in
+ * ns_per_cell_step (host, PDM1_NUM_TILES, may be NULL). */
 #define PDM1_NUM_TILES 3
 int pdm1_tile_shape(int tile_id, int *tx, int *ty, int *tz);
 int pdm1_plan_set_tile(pdm1_plan *plan, int tile_id);

@@ -118,7 +118,8 @@ class Accel:
     graph_chunk_steps: int = 32
     # Tile shape of the stage kernels: None = 4x8x8, a shape (x, y, z) among
     # TILE_SHAPES, or "auto" = the fastest shape measured on the plan's problem
-    # by the autotuner (cached per precision, grid and beam count).
+    # by the autotuner (cached per precision, grid and beam count).  A grid whose
+    # 4x4x4 tiles fit one wave of CTAs runs on those under every setting.
     tile: tuple[int, int, int] | str | None = None
     # Learned moving box (learned_box.BoxModel); None = the fixed heuristic box.
     # Needs numerics.moving_active_domain.
