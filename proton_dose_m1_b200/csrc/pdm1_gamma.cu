@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <exception>
 #include <vector>
 
 namespace {
@@ -126,21 +127,28 @@ extern "C" int pdm1_gamma(const double *dose_ref, const double *dose_eval, int n
     // candidate offsets on the interpolation lattice inside the search sphere, by distance
     const double h = distance_mm / interp_fraction;
     const double R = (max_gamma > 0 ? max_gamma : 1.0) * distance_mm;
-    const int m = (int)std::floor(R / h + 1e-9);
-    // (sorted within the shells of equal a^2 + b^2 + c^2, whose distances differ by rounding only)
-    std::vector<std::vector<Offset>> shells(3 * (size_t)m * m + 1);
-    for (int a = -m; a <= m; ++a)
-        for (int b = -m; b <= m; ++b)
-            for (int c = -m; c <= m; ++c) {
-                double x = a * h, y = b * h, z = c * h;
-                double r2 = x * x + y * y + z * z;
-                if (r2 <= R * R * (1.0 + 1e-12))
-                    shells[(size_t)(a * a + b * b + c * c)].push_back({x, y, z, r2 / (distance_mm * distance_mm)});
-            }
+    const double cells = std::floor(R / h + 1e-9);
+    const int m = cells >= 0.0 && cells < 2147483647.0 ? (int)cells : -1;
+    // (sorted within the shells of equal a^2 + b^2 + c^2, whose distances differ by rounding only);
+    // a radius that the lattice cannot count (infinite: m < 0) has no candidates
     std::vector<Offset> offs;
-    for (auto &s : shells) {
-        std::stable_sort(s.begin(), s.end(), [](const Offset &p, const Offset &q) { return p.d2 < q.d2; });
-        offs.insert(offs.end(), s.begin(), s.end());
+    try {
+        std::vector<std::vector<Offset>> shells(m < 0 ? 0 : 3 * (size_t)m * m + 1);
+        for (int a = -m; a <= m; ++a)
+            for (int b = -m; b <= m; ++b)
+                for (int c = -m; c <= m; ++c) {
+                    double x = a * h, y = b * h, z = c * h;
+                    double r2 = x * x + y * y + z * z;
+                    if (r2 <= R * R * (1.0 + 1e-12))
+                        shells[(size_t)((long long)a * a + (long long)b * b + (long long)c * c)].push_back(
+                            {x, y, z, r2 / (distance_mm * distance_mm)});
+                }
+        for (auto &s : shells) {
+            std::stable_sort(s.begin(), s.end(), [](const Offset &p, const Offset &q) { return p.d2 < q.d2; });
+            offs.insert(offs.end(), s.begin(), s.end());
+        }
+    } catch (const std::exception &) {   // more candidates than memory holds: no C++ exception leaves a C entry
+        return PDM1_ERR_ARGUMENT;
     }
     Offset *d_off = nullptr;
     unsigned long long *d_counts = nullptr;
