@@ -34,9 +34,10 @@ struct Offset {
 __device__ __forceinline__ double trilinear(const double *D, int nx, int ny, int nz, double fi, double fj,
                                             double fk) {
     int i = (int)floor(fi), j = (int)floor(fj), k = (int)floor(fk);
-    i = i < 0 ? 0 : (i > nx - 2 ? nx - 2 : i);
-    j = j < 0 ? 0 : (j > ny - 2 ? ny - 2 : j);
-    k = k < 0 ? 0 : (k > nz - 2 ? nz - 2 : k);
+    // the lower corner of the cell; an axis of one cell has corner 0 only
+    i = max(min(i, nx - 2), 0);
+    j = max(min(j, ny - 2), 0);
+    k = max(min(k, nz - 2), 0);
     double ti = nx > 1 ? fi - i : 0.0, tj = ny > 1 ? fj - j : 0.0, tk = nz > 1 ? fk - k : 0.0;
     int i1 = nx > 1 ? i + 1 : i, j1 = ny > 1 ? j + 1 : j, k1 = nz > 1 ? k + 1 : k;
     auto at = [&](int a, int b, int c) { return D[((size_t)a * ny + b) * nz + c]; };
