@@ -298,7 +298,11 @@ __device__ __forceinline__ void stage_tile(const StageArgs &a, const ConfigDev &
                 z(2) = T(3.0) * ui - T(2.5) * u0 + T(0.5) * u1;
                 z(1) = T(9.0) * ui - T(10.5) * u0 + T(2.5) * u1;
             }
-            if constexpr (kNear) out_of_range |= !(weno_range(z(0)) && weno_range(z(1)) && weno_range(z(2)));
+            if constexpr (kNear) {   // the ghosts just written; what lies in the others is an earlier tile's
+                const int first = cf.spatial == PDM1_SPATIAL_WENO_Z ? 0 : (cf.spatial == PDM1_SPATIAL_FIRST_ORDER ? 2 : 1);
+#pragma unroll
+                for (int kk = 0; kk < 3; ++kk) out_of_range |= kk >= first && !weno_range(z(kk));
+            }
         }
         if constexpr (kNear) ieee = __syncthreads_or(out_of_range) != 0;
         else __syncthreads();
