@@ -1291,8 +1291,11 @@ int create_plan(const pdm1_problem *problem, const pdm1_beam *beams, int nbeams,
     if (ok) {   // d_tile_off lends the word the ids are checked into; the march clears it
         unsigned *mask = reinterpret_cast<unsigned *>(pl->d_tile_off);
         ok = cudaMemset(mask, 0, sizeof *mask) == cudaSuccess;
+        (void)cudaGetLastError();   // start from a clean launch-error state
         ids_kernel<<<(int)std::min<size_t>((N + 255) / 256, (size_t)8 * pl->sms), 256>>>(pl->d_ids, N, p.n_materials, mask);
-        ok = ok && cudaMemcpy(&cf.present, mask, sizeof cf.present, cudaMemcpyDeviceToHost) == cudaSuccess;
+        ok = ok && cudaGetLastError() == cudaSuccess &&
+             cudaMemcpy(&cf.present, mask, sizeof cf.present, cudaMemcpyDeviceToHost) == cudaSuccess &&
+             cf.present != 0u;   // every cell sets a bit: none, and the ids were not looked at
         if (ok && (cf.present & 0x80000000u)) return fail(set_error(PDM1_ERR_ARGUMENT, "material id out of range"));
     }
     ok = ok &&
