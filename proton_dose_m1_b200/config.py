@@ -118,8 +118,9 @@ class Accel:
     graph_chunk_steps: int = 32
     # Tile shape of the stage kernels: None = 4x8x8, a shape (x, y, z) among
     # TILE_SHAPES, or "auto" = the fastest shape measured on the plan's problem
-    # by the autotuner (cached per precision, grid and beam count).  A grid whose
-    # 4x4x4 tiles fit one wave of CTAs runs on those under every setting.
+    # by the autotuner (cached per precision, grid, one beam or a field, and full domain
+    # or moving box).  A plan whose grids of all beams fit one wave of CTAs in 4x4x4 tiles
+    # runs on those under every setting; it is not measured.
     tile: tuple[int, int, int] | str | None = None
     # Learned moving box (learned_box.BoxModel); None = the fixed heuristic box.
     # Needs numerics.moving_active_domain.

@@ -1555,6 +1555,11 @@ int pdm1_plan_set_staging(pdm1_plan *pl, int bulk) {
 int pdm1_plan_autotune(pdm1_plan *pl, int steps, int *best_tile, double *ns_per_cell_step, pdm1_stream_t stream) {
     if (!pl) return set_error(PDM1_ERR_ARGUMENT, "plan is NULL");
     if (steps < 1) return set_error(PDM1_ERR_ARGUMENT, "steps must be >= 1");
+    if (pl->cf.tile_id == kSmallTileId) {   // 4x4x4 under every setting: nothing to measure
+        if (best_tile) *best_tile = 0;
+        for (int id = 0; ns_per_cell_step && id < kNumTiles; ++id) ns_per_cell_step[id] = 0.0;
+        return PDM1_OK;
+    }
     const size_t N = (size_t)pl->p.nx * pl->p.ny * pl->p.nz;
     double *U = nullptr, *dose = nullptr, *energies = nullptr;
     auto release = [&]() { cudaFree(U); cudaFree(dose); cudaFree(energies); };

@@ -134,6 +134,8 @@ def _apply_tile(config, handle, shape, n_beams) -> None:
         ns = (C.c_double * _native.NUM_TILES)()
         _native.check(_native.lib().pdm1_plan_autotune(handle, AUTOTUNE_STEPS, C.byref(best), ns,
                                                        C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+        if not any(ns):   # a plan on 4x4x4 tiles measures nothing: the choice is left to larger ones
+            return
         _TILE_CACHE[key] = (int(best.value), [float(v) for v in ns])
     _native.check(_native.lib().pdm1_plan_set_tile(handle, _TILE_CACHE[key][0]))
 
