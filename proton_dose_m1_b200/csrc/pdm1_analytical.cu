@@ -261,25 +261,29 @@ extern "C" int pdm1_analytical_csda_dose(const pdm1_problem *p, int energy_point
         col_of[xy] = found;
     }
     const int ncol = (int)first.size();
-    double *d_blob = nullptr, *d_tab = nullptr, *d_invS = nullptr, *d_lost = nullptr, *d_rho = nullptr, *d_sp = nullptr;
-    int *d_cm = nullptr, *d_colof = nullptr;
-    int32_t *d_ids = nullptr;
-    RangeView *d_tabs = nullptr;
-    TableView *d_views = nullptr;
-    auto release = [&]() {   // back to the pool: nothing of this call may still use them
-        cudaStreamSynchronize(stream);
-        for (void *q : {(void *)d_blob, (void *)d_tab, (void *)d_invS, (void *)d_lost, (void *)d_rho, (void *)d_sp,
-                        (void *)d_cm, (void *)d_colof, (void *)d_ids, (void *)d_tabs, (void *)d_views})
-            pool_free(q);
-    };
-    auto get = [](auto *&q, size_t n) { return pool_malloc((void **)&q, n * sizeof(*q)) == cudaSuccess; };
-    bool ok = get(d_blob, 2 * (size_t)nm * range_points) && get(d_invS, (size_t)nm * range_points) &&
-              get(d_tab, tables.size()) && get(d_views, nm) && get(d_lost, (size_t)ncol * nz) && get(d_rho, nm) &&
-              get(d_sp, NXY) && get(d_cm, col_mats.size()) && get(d_colof, NXY) && get(d_ids, N) && get(d_tabs, nm);
-    if (!ok) {
-        release();
+    // one block for the call's buffers
+    unsigned char *block = nullptr;
+    size_t used = 0;
+    auto part = [&](size_t bytes) { const size_t at = used; used = (at + bytes + 255) & ~size_t(255); return at; };
+    const size_t o_blob = part(2 * (size_t)nm * range_points * sizeof(double));
+    const size_t o_invS = part((size_t)nm * range_points * sizeof(double));
+    const size_t o_tab = part(tables.size() * sizeof(double)), o_views = part(nm * sizeof(TableView));
+    const size_t o_lost = part((size_t)ncol * nz * sizeof(double)), o_rho = part(nm * sizeof(double));
+    const size_t o_sp = part(NXY * sizeof(double)), o_cm = part(col_mats.size() * sizeof(int));
+    const size_t o_colof = part(NXY * sizeof(int)), o_ids = part(N * sizeof(int32_t));
+    const size_t o_tabs = part(nm * sizeof(RangeView));
+    if (pool_malloc_workspace((void **)&block, used) != cudaSuccess)
         return report_error(PDM1_ERR_CUDA, "pdm1_analytical_csda_dose: cudaMalloc failed");
-    }
+    auto release = [&]() {   // back to the pool: nothing of this call may still use it
+        cudaStreamSynchronize(stream);
+        pool_free(block);
+    };
+    double *d_blob = (double *)(block + o_blob), *d_invS = (double *)(block + o_invS), *d_tab = (double *)(block + o_tab);
+    double *d_lost = (double *)(block + o_lost), *d_rho = (double *)(block + o_rho), *d_sp = (double *)(block + o_sp);
+    int *d_cm = (int *)(block + o_cm), *d_colof = (int *)(block + o_colof);
+    int32_t *d_ids = (int32_t *)(block + o_ids);
+    TableView *d_views = (TableView *)(block + o_views);
+    RangeView *d_tabs = (RangeView *)(block + o_tabs);
     size_t at = 0;
     for (int m = 0; m < nm; ++m) {
         sp[m].E = d_tab + at;

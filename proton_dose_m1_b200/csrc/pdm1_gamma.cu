@@ -151,13 +151,11 @@ extern "C" int pdm1_gamma(const double *dose_ref, const double *dose_eval, int n
     } catch (const std::exception &) {   // more candidates than memory holds: no C++ exception leaves a C entry
         return PDM1_ERR_ARGUMENT;
     }
-    Offset *d_off = nullptr;
-    unsigned long long *d_counts = nullptr;
-    if (pdm1::pool_malloc((void **)&d_off, offs.size() * sizeof(Offset)) != cudaSuccess ||
-        pdm1::pool_malloc((void **)&d_counts, 2 * sizeof(unsigned long long)) != cudaSuccess) {
-        pdm1::pool_free(d_off);
+    unsigned long long *d_counts = nullptr;   // the two counts, then the candidates
+    const size_t head = 256;
+    if (pdm1::pool_malloc_workspace((void **)&d_counts, head + offs.size() * sizeof(Offset)) != cudaSuccess)
         return PDM1_ERR_CUDA;
-    }
+    Offset *d_off = (Offset *)((unsigned char *)d_counts + head);
     cudaMemcpyAsync(d_off, offs.data(), offs.size() * sizeof(Offset), cudaMemcpyHostToDevice, stream);
     cudaMemsetAsync(d_counts, 0, 2 * sizeof(unsigned long long), stream);
     double dD = dose_percent / 100.0 * global_normalisation;
@@ -170,8 +168,7 @@ extern "C" int pdm1_gamma(const double *dose_ref, const double *dose_eval, int n
     unsigned long long counts[2] = {0, 0};
     cudaError_t e = cudaMemcpyAsync(counts, d_counts, sizeof counts, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e != cudaSuccess) cudaStreamSynchronize(stream);   // nothing of this call still uses the blocks
-    pdm1::pool_free(d_off);
+    if (e != cudaSuccess) cudaStreamSynchronize(stream);   // nothing of this call still uses the block
     pdm1::pool_free(d_counts);
     if (e != cudaSuccess) return PDM1_ERR_CUDA;
     if (pass_rate_out) *pass_rate_out = counts[1] ? 100.0 * (double)counts[0] / (double)counts[1] : NAN;

@@ -10,6 +10,7 @@
 // the request retried.  pdm1_pool_release() returns the cache to the driver.
 #include <cuda_runtime.h>
 
+#include <cstdint>
 #include <map>
 #include <mutex>
 #include <unordered_map>
@@ -109,6 +110,12 @@ cudaError_t pool_malloc(void **ptr, size_t bytes) {
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     return acquire(ptr, bytes, device);
+}
+
+cudaError_t pool_malloc_workspace(void **ptr, size_t bytes) {
+    size_t r = 512;
+    while (r < bytes && r <= SIZE_MAX / 2) r <<= 1;
+    return pool_malloc(ptr, r < bytes ? bytes : r);
 }
 
 cudaError_t pool_malloc_host(void **ptr, size_t bytes) { return acquire(ptr, bytes, kHostDevice); }
