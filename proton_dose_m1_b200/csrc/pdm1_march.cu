@@ -1056,6 +1056,11 @@ int set_smem_attributes() {
     return PDM1_OK;
 }
 
+// A copy from pageable memory returns once it is staged, and a memset at once: the device
+// may not have them yet.  A march on a stream that does not wait for the legacy stream must
+// not start ahead of the plan's uploads.
+cudaError_t uploads_done() { return cudaStreamSynchronize(cudaStreamLegacy); }
+
 int device_error_status(int error) {
     if (error & ERR_DEV_RANGE) return set_error(PDM1_ERR_RANGE, "energy outside a coefficient table during the march");
     if (error & ERR_DEV_MAXSTEPS) return set_error(PDM1_ERR_MAX_STEPS, "energies buffer shorter than the march");
@@ -1306,7 +1311,7 @@ int create_plan(const pdm1_problem *problem, const pdm1_beam *beams, int nbeams,
     for (int b = 0; ok && b < nbeams; ++b)
         ok = cudaMemcpy(pl->d_spatial + (size_t)b * NXY, beams[b].inflow_spatial, NXY * sizeof(double),
                         cudaMemcpyHostToDevice) == cudaSuccess;
-    if (!ok) return fail(set_error(PDM1_ERR_CUDA, "plan upload failed"));
+    if (!ok || uploads_done() != cudaSuccess) return fail(set_error(PDM1_ERR_CUDA, "plan upload failed"));
     *out = pl;
     return PDM1_OK;
 }
@@ -1524,6 +1529,7 @@ int pdm1_plan_set_tile(pdm1_plan *pl, int tile_id) {
         bd.init_box = make_domain(o.i0, o.j0, o.k0, o.nx, o.ny, o.nz, o.inflow, t);
     }
     CUDA_TRY(cudaMemcpy(pl->d_beams, pl->h_beams.data(), pl->h_beams.size() * sizeof(BeamDev), cudaMemcpyHostToDevice));
+    CUDA_TRY(uploads_done());
     return PDM1_OK;
 }
 
@@ -1541,6 +1547,7 @@ int pdm1_plan_set_schedule(pdm1_plan *pl, const double *energies, int n) {
     if (n == 0) return PDM1_OK;
     CUDA_TRY(pool_malloc((void **)&pl->d_schedule, (size_t)n * sizeof(double)));
     CUDA_TRY(cudaMemcpy(pl->d_schedule, energies, (size_t)n * sizeof(double), cudaMemcpyHostToDevice));
+    CUDA_TRY(uploads_done());
     pl->cf.schedule = pl->d_schedule;
     pl->cf.n_schedule = n;
     return PDM1_OK;
@@ -1610,6 +1617,7 @@ int pdm1_plan_set_box_model(pdm1_plan *pl, const pdm1_box_model *model) {
     if (rc) return rc;
     if (!pl->d_model) CUDA_TRY(pool_malloc((void **)&pl->d_model, sizeof(BoxModelDev)));
     CUDA_TRY(cudaMemcpy(pl->d_model, &h, sizeof h, cudaMemcpyHostToDevice));
+    CUDA_TRY(uploads_done());
     pl->cf.learned = 1;
     pl->cf.model = pl->d_model;
     return PDM1_OK;
