@@ -1719,6 +1719,8 @@ int pdm1_energy_step(pdm1_plan *pl, const double *U, double energy, double *dE_o
 int pdm1_advance(pdm1_plan *pl, double *U, double energy, double dE, double *edep, pdm1_stream_t stream_) {
     (void)cudaGetLastError();
     if (!pl || !U || !edep || !(dE > 0.0) || pl->nbeams != 1) return set_error(PDM1_ERR_ARGUMENT, "dE must be positive.");
+    if (pl->cap < (size_t)pl->p.nx * pl->p.ny * pl->p.nz)
+        return set_error(PDM1_ERR_ARGUMENT, "the plan's buffers hold a moving box, not the full grid");
     cudaStream_t stream = (cudaStream_t)stream_;
     int rc = check_energy_range(pl, energy, energy - dE);
     if (rc) return rc;
