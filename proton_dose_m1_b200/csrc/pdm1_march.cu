@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -1896,7 +1897,7 @@ extern "C" int pdm1_march_noalloc(const pdm1_problem *problem, double *U, double
     const size_t o_st = off; off = align256(off + sizeof(MarchState));
     const size_t o_bm = off; off = align256(off + sizeof(BeamDev));
     const size_t o_to = off; off = align256(off + (2 + kTileCounters) * sizeof(int));
-    const size_t o_sm = off; off = align256(off + sizeof(MarchSummary));
+    const size_t o_sm = off; off = align256(off + offsetof(MarchSummary, begin_ns));   // its stages are not timed
     size_t o_tab[kMaxMat][3];
     for (int m = 0; m < p.n_materials; ++m) {
         const pdm1_table *tabs[3] = {&p.materials[m].stopping_power, &p.materials[m].transport,
