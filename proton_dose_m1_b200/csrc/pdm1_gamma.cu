@@ -50,12 +50,25 @@ __device__ __forceinline__ double trilinear(const double *D, int nx, int ny, int
     return c0 * (1.0 - ti) + c1 * ti;
 }
 
-// A CTA per 256 voxels: the voxels at or above the cutoff are listed in shared
-// memory and searched by one warp each, 32 candidates at a time.  A voxel's gamma is the
+// Squared gamma of the candidate `ofs` of voxel (i, j, k) with dose dr; infinite outside the grid.
+__device__ __forceinline__ double candidate(const Offset &ofs, const double *eval, int nx, int ny, int nz, double hx,
+                                            double hy, double hz, int i, int j, int k, double dr, double inv_dd2) {
+    const double fi = i + ofs.dx / hx, fj = j + ofs.dy / hy, fk = k + ofs.dz / hz;
+    if (fi < 0.0 || fi > nx - 1 || fj < 0.0 || fj > ny - 1 || fk < 0.0 || fk > nz - 1) return INFINITY;
+    const double de = trilinear(eval, nx, ny, nz, fi, fj, fk) - dr;
+    return ofs.d2 + de * de * inv_dd2;
+}
+
+// A CTA per 256 voxels: each thread takes the nearest candidate (the voxel itself); the
+// voxels at or above the cutoff that it does not pass are listed in shared memory and
+// searched by one warp each, 32 candidates at a time.  A voxel's gamma is the
 // first candidate's that passes (skip_once_passed) or the smallest of all that are nearer
 // than it, in whichever way they are evaluated; a thread per voxel walked up to 5575
 // candidates in turn, and the few voxels that fail held the kernel for them (80x80x400 at
-// 0.5 mm, 1 %/1 mm, whole call: 1.7-5.6 ms by the share that fails -> 0.5 ms).
+// 0.5 mm, 1 %/1 mm, whole call: 1.7-5.6 ms by the share that fails -> 0.5 ms).  Where nearly
+// all pass at the first candidate, as two close doses without a cutoff do, a warp for each of
+// them took 14 ms on 256x256x320, a thread 1.2 ms (2 to 32 candidates by the thread: no
+// faster).
 constexpr int kGammaThreads = 256;
 __global__ void __launch_bounds__(kGammaThreads) gamma_kernel(const double *ref, const double *eval, int nx, int ny,
                                                               int nz, double hx, double hy, double hz,
@@ -68,13 +81,27 @@ __global__ void __launch_bounds__(kGammaThreads) gamma_kernel(const double *ref,
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) n_list = 0;
     __syncthreads();
+    unsigned pass = 0, valid = 0;
+    auto finish = [&](size_t o, double best) {
+        double g = sqrt(best);
+        if (g > max_gamma) g = max_gamma > 0.0 ? INFINITY : g;
+        gamma[o] = g;
+        ++valid;
+        pass += g <= 1.0;
+    };
     const size_t mine = base + threadIdx.x;
     if (mine < N) {
-        if (ref[mine] >= cutoff) list[atomicAdd(&n_list, 1)] = threadIdx.x;
-        else gamma[mine] = NAN;
+        const double dr = ref[mine];
+        if (dr >= cutoff) {
+            const int k = (int)(mine % nz), j = (int)((mine / nz) % ny), i = (int)(mine / ((size_t)nz * ny));
+            const double g2 = n_off > 0 ? candidate(off[0], eval, nx, ny, nz, hx, hy, hz, i, j, k, dr, inv_dd2) : INFINITY;
+            if (skip_once_passed && g2 <= 1.0) finish(mine, g2);
+            else list[atomicAdd(&n_list, 1)] = threadIdx.x;
+        } else {
+            gamma[mine] = NAN;
+        }
     }
     __syncthreads();
-    unsigned long long pass = 0, valid = 0;
     for (int v = threadIdx.x >> 5; v < n_list; v += kGammaThreads / 32) {
         const size_t o = base + list[v];
         const double dr = ref[o];
@@ -86,11 +113,7 @@ __global__ void __launch_bounds__(kGammaThreads) gamma_kernel(const double *ref,
             if (q < n_off) {
                 const Offset ofs = off[q];
                 d2 = ofs.d2;
-                const double fi = i + ofs.dx / hx, fj = j + ofs.dy / hy, fk = k + ofs.dz / hz;
-                if (!(fi < 0.0 || fi > nx - 1 || fj < 0.0 || fj > ny - 1 || fk < 0.0 || fk > nz - 1)) {
-                    double de = trilinear(eval, nx, ny, nz, fi, fj, fk) - dr;
-                    g2 = ofs.d2 + de * de * inv_dd2;
-                }
+                g2 = candidate(ofs, eval, nx, ny, nz, hx, hy, hz, i, j, k, dr, inv_dd2);
             }
             if (__shfl_sync(0xffffffffu, d2, 0) >= best) break;   // farther points cannot win
             const unsigned passed = __ballot_sync(0xffffffffu, skip_once_passed && g2 <= 1.0);
@@ -101,15 +124,13 @@ __global__ void __launch_bounds__(kGammaThreads) gamma_kernel(const double *ref,
             for (int w = 16; w > 0; w >>= 1) g2 = fmin(g2, __shfl_xor_sync(0xffffffffu, g2, w));
             best = fmin(best, g2);
         }
-        double g = sqrt(best);
-        if (g > max_gamma) g = max_gamma > 0.0 ? INFINITY : g;
-        if (lane == 0) gamma[o] = g;
-        ++valid;
-        pass += g <= 1.0;
+        if (lane == 0) finish(o, best);
     }
+    pass = __reduce_add_sync(0xffffffffu, pass);
+    valid = __reduce_add_sync(0xffffffffu, valid);
     if (lane == 0 && valid) {
-        atomicAdd(&counts[0], pass);
-        atomicAdd(&counts[1], valid);
+        atomicAdd(&counts[0], (unsigned long long)pass);
+        atomicAdd(&counts[1], (unsigned long long)valid);
     }
 }
 
