@@ -44,7 +44,7 @@ def test_unbounded_search_has_no_candidates(distance, fraction, max_gamma):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(1, 9, 8), (7, 1, 8), (7, 9, 1), (1, 1, 12), (1, 12, 1), (12, 1, 1), (1, 1, 1), (2, 1, 2)])
-def test_axis_of_one_cell_equals_checker(shape):
+def test_axis_of_one_cell_equals_oracle(shape):
     """Doses of one layer or one line: the interpolation stays on their only layer."""
     r = np.random.default_rng(sum(shape))
     ref = 1.0 + 0.02 * r.random(shape)
